@@ -170,6 +170,11 @@ class _Flow:
         flow, kind = _flow(case), case["kind"]
         with tempfile.TemporaryDirectory() as d:
             s = self.solver = Solver.from_case(flow, d, storage=case["storage"])
+        self.free = ctypes.CDLL(None).free
+        self.free.argtypes = [ctypes.c_void_p]
+        members = [getattr(s.fluid, name) for name, _ in abi.FluidT._fields_]
+        self.arrays = [m for m in members if isinstance(m, abi.ArrayT)]
+        self.arrays += [a for m in members if isinstance(m, abi.ArrayT * 3) for a in m]
         s.set_coherence(abi.PIN_HOST | (0 if kind == "integrate" else abi.NO_COHERENCE))
         for n, v in _initial(case, seed).items():
             torch.from_numpy(s.field(n))[1:-1, 1:-1].copy_(v)
@@ -192,12 +197,8 @@ class _Flow:
         if getattr(self, "solver", None) is None:
             return
         self.solver.release()
-        free = ctypes.CDLL(None).free
-        free.argtypes = [ctypes.c_void_p]
-        for name, kind in abi.FluidT._fields_:
-            member = getattr(self.solver.fluid, name)
-            for a in (member if kind is abi.ArrayT * 3 else [member] if kind is abi.ArrayT else []):
-                free(a.data)
+        for a in self.arrays:
+            self.free(a.data)
 
 
 def prepare(case, seed):
