@@ -93,7 +93,7 @@ def draw(rng):
         two = all(n & (n - 1) == 0 for n in (ny, nz))
         if cells <= (4_000_000 if kind == "integrate" else 40_000_000 if two else 16_000_000):
             break
-    steps = 4 if kind == "integrate" else max(2, min(32, int(1.5e8 / cells)))
+    steps = 4 if kind == "integrate" else max(2, min(32, int((1.5e8 if two else 5e7) / cells)))
     curved = rng.random() < 0.75
     implicit = "x" if curved else rng.choice(("xyz", "xyz", "x"))
     if rng.random() < 0.1:
