@@ -410,20 +410,21 @@ static int build_tables(Ctx & c, const domain_t * d) {
   double * dP = dalloc(c, P.size());
   if (!dP) return fail("cudaMalloc failed");
   CK(cudaMemcpy(dP, P.data(), P.size() * sizeof(double), cudaMemcpyHostToDevice));
-  // factor rows cover every element a solving warp touches (32 lanes x
-  // elements per lane) and start on 16-byte boundaries for paired loads
-  const size_t LX = ((std::max(L, (size_t)32 * predict_warps(nx)) + 1) / 2) * 2;
+  c.xf.single = c.sb == 4;
+  c.xf.ne = c.xf.single ? predict_warps32(nx) : predict_warps(nx);
+  const size_t LX = (size_t)32 * c.xf.ne;   // every element a solving warp touches
   c.xf.stride = LX;
-  c.xf.ne = predict_warps(nx);   // the march kernel solves with E = its warp count elements per lane
   for (int v = 0; v < 4; v++) {
     c.xf.n[v] = (v == VUX) ? nx - 1 : nx;
     c.xf.lap_l[v] = dP + (size_t)v * 6 * L;
     c.xf.lap_c[v] = dP + (size_t)v * 6 * L + L;
     c.xf.lap_u[v] = dP + (size_t)v * 6 * L + 2 * L;
   }
-  c.xf.lo = dalloc(c, 12 * LX);
+  c.xf.f = dalloc(c, 12 * LX);
+  c.xf.g = dalloc(c, 12 * LX);
   c.xf.w = dalloc(c, 12 * LX);
-  c.xf.v = dalloc(c, 12 * LX);
+  c.xf.scan = dalloc(c, 12 * XSCAN_ROWS * 32);
+  if (!c.xf.f || !c.xf.g || !c.xf.w || !c.xf.scan) return fail("cudaMalloc of the radial factors failed");
   if (c.bc.implicit[1] || c.bc.implicit[2]) {
     YZFactors & yf = c.yf;
     yf.max_i = nx;

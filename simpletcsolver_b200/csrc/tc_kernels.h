@@ -118,17 +118,25 @@ struct Coefs {
   double inv_hz;
 };
 
-// Radial Thomas factors for the three substeps x four variables.
+// Radial Thomas factors for the three substeps x four variables (rows of each
+// kind: [12][stride]; element e of a row at (e % ne) 32 + e / ne, so that the ne
+// elements a lane of the solving warp owns, e = lane ne + m, are read with one
+// coalesced load per m; entries from n on are zero).
+constexpr int XSCAN_ROWS = 10;   // scan levels forward, then backward
 struct XFactors {
   int n[4];                 // nx-1 for ux, nx otherwise
-  size_t stride;            // >= nx
+  size_t stride;            // 32 ne
   const double * lap_l[4];  // per-variable Laplacian coefficients, packed e = i - i0
   const double * lap_c[4];
   const double * lap_u[4];
-  double * lo;              // [12][stride], element e of a row at (e % ne) 32 + e / ne: the
-  double * w;               // ne elements a lane of the solving warp owns (e = lane ne + m)
-  double * v;               // are read with one coalesced load per m
+  double * f;               // -l_e w_{e-1}
+  double * g;               // -u_e w_{e+1}
+  double * w;               // 1 / pivot
+  double * scan;            // [12][XSCAN_ROWS][32] products of f (g) over the lanes a scan level spans
   int ne;                   // elements per lane of the radial solves (warps of the predict kernel)
+  // FP32-storage contexts keep the rows of tc_march_f32.cu: f holds l_e (l_0 = 0),
+  // g the back-substitution factor u_e w_e (0 in the last row); no scan products
+  bool single;
 };
 
 // Periodic y / z factors (planar configuration with implicit y and z).
@@ -216,6 +224,8 @@ struct DeltaSet {
 };
 enum { PREDICT_APPLY = 0, PREDICT_DELTA = 1 };
 int predict_warps(int nx);
+int predict_warps32(int nx);   // the same for FP32-storage contexts
+int march_planes(long long columns, int nz, int per_sm);
 // marching form of the predict stage (tc_march.cu); sets ST_TIMEOUT in
 // *status if a plane's copy does not arrive within its wait limit
 void launch_predict_march(const Geo & g, const Bc & bc, const Coefs & cf, const XFactors & xf, double nu,
@@ -223,6 +233,13 @@ void launch_predict_march(const Geo & g, const Bc & bc, const Coefs & cf, const 
                           const DeltaSet & ds, const double * dtp, int rkstep, int mode, unsigned * status,
                           cudaStream_t st);
 void march_smem_limits();
+// the same for FP32-storage contexts (tc_march_f32.cu)
+void launch_predict_march32(const Geo & g, const Bc & bc, const Coefs & cf, const XFactors & xf, double nu,
+                            double kappa, const FieldBufs & in, const FieldBufs & out, const SrcBufs & ss,
+                            const DeltaSet & ds, const double * dtp, int rkstep, int mode, unsigned * status,
+                            cudaStream_t st);
+void launch_xsolve32(const Geo & g, const XFactors & xf, int rkstep, const DeltaSet & ds, cudaStream_t st);
+void march32_smem_limits();
 // radial implicit solves of the delta buffers, lines of up to 1024 points
 // (after the predict's tile mode, nx > 256)
 void launch_xsolve(const Geo & g, const XFactors & xf, int rkstep, const DeltaSet & ds, cudaStream_t st);

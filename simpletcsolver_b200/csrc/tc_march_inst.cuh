@@ -1,0 +1,43 @@
+// Definitions behind tc_march_launch.cuh, for the instantiating files.
+#pragma once
+#include <atomic>
+
+#include "tc_march_launch.cuh"
+
+namespace tcgpu {
+namespace march {
+
+template <int NW, int PAIRS, int NG, int IMPL, class T, bool TILE>
+void launch_one(Args<T> A, const double * dtp, cudaStream_t st) {
+  using L = Layout<NW, PAIRS, NG, T>;
+  const long long columns = (long long)((A.g.ny + L::JT - 1) / L::JT) * (TILE ? (A.g.nx + L::NT - 1) / L::NT : 1);
+  A.KC = march_planes(columns, A.g.nz, 1);
+  auto kernel = predict_kernel<NW, PAIRS, NG, IMPL, T, TILE>;
+  static std::atomic<unsigned> allowed{0};   // devices (bit) that know this instance's shared memory
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const unsigned bit = 1u << (dev & 31);
+  if (!(allowed.load(std::memory_order_relaxed) & bit)) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES) != cudaSuccess) return;
+    allowed.fetch_or(bit, std::memory_order_relaxed);
+  }
+  kernel<<<(unsigned)(columns * (A.g.nz / A.KC)), L::THREADS, L::BYTES, st>>>(A, dtp);
+}
+
+// warps per line by its length, and as many line pairs as make 12 to 16 field warps
+#ifndef TC_MARCH_INSTANCES
+#define TC_MARCH_INSTANCES(X) X(1, 4, 1) X(2, 4, 1) X(3, 2, 2) X(4, 2, 1) X(6, 1, 2) X(8, 1, 1)
+#endif
+
+template <int IMPL, class T>
+void launch(Args<T> A, bool tiles, const double * dtp, cudaStream_t st) {
+  if constexpr (IMPL < 0 || IMPL == 1)
+    if (tiles) return launch_one<8, 1, 1, IMPL, T, true>(A, dtp, st);
+  switch (predict_warps(A.g.nx)) {
+#define X(NW, PAIRS, NG) case NW: return launch_one<NW, PAIRS, NG, IMPL, T, false>(A, dtp, st);
+    TC_MARCH_INSTANCES(X)
+#undef X
+  }
+}
+}  // namespace march
+}  // namespace tcgpu

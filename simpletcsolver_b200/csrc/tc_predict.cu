@@ -11,51 +11,113 @@
 namespace tcgpu {
 
 // ------------------------------------------------------------ Thomas factors
-// One thread per (substep, variable, direction): the forward-elimination
-// factors of gtsv (src/tdm.c:24-44) for (I - pf L) with
+// One block per (substep, variable): the factors of gtsv (src/tdm.c:24-44) for
+// (I - pf L) with
 //   l = -pf lap.l, c = 1 - pf lap.c, u = -pf lap.u   (predict/linear_system.c:26-33)
 // pf = 0.5 gamma dt diffusivity, doubled for the "diagonal" component
-// (ux-x ux.c:502, uy-y uy.c:541, uz-z uz.c:451, t-y t.c:348).
-// Output per line family: lo[n] = l (lo[0] = 0), w[n] (w[0] = 1/c[0],
-// w[i] = 1/(c - l v)), v[n] (v[n-1] = 0), so every row of the forward sweep
-// reads q = w (r - l q_prev). Entries from n on stay zero. Rows are stored
-// interleaved for the warp that solves them (XFactors::ne).
-__global__ void xfactor_kernel(XFactors xf, const double * __restrict__ dtp, double nu, double kappa) {
-  const int tid = threadIdx.x;
-  if (tid >= 12) return;
-  const int rk = tid / 4, var = tid % 4;
+// (ux-x ux.c:502, uy-y uy.c:541, uz-z uz.c:451, t-y t.c:348), in the form the
+// solves use (XFactors). The pivots c_e - l_e u_{e-1} / pivot_{e-1} are ratios of
+// successive leading minors, theta_e = c_e theta_{e-1} - l_e u_{e-1} theta_{e-2},
+// whose recurrence is two multiply-adds an element instead of a division; the
+// divisions theta_{e-1} / theta_e then run in parallel. Every pair of minors is
+// scaled by a power of two (exact) when it leaves [2^-256, 2^256].
+// Bound: the serial recurrence (256 elements, two dependent FP64 operations
+// each). The former single block, one thread per line with a division and three
+// global loads per element: 108 us at nx = 256, on every step's critical path.
+constexpr int XF_MAX = 1024;   // longest radial line
+__global__ void __launch_bounds__(256) xfactor_kernel(XFactors xf, const double * __restrict__ dtp, double nu, double kappa) {
+  __shared__ double sl[XF_MAX], sc[XF_MAX], su[XF_MAX];   // l u_{e-1}; c, then theta_e; theta_{e-1}, then w
+  const int rv = blockIdx.x, rk = rv / 4, var = rv % 4, tid = threadIdx.x;
   const double dt = *dtp;
   const double diff = (var == VT) ? kappa : nu;
   double pf = 0.5 * rk_gamma(rk) * dt * diff;
   if (var == VUX) pf = 2. * pf;
-  const int n = xf.n[var];
-  const double * ll = xf.lap_l[var];
-  const double * lc = xf.lap_c[var];
-  const double * lu = xf.lap_u[var];
-  double * lo = xf.lo + (size_t)(rk * 4 + var) * xf.stride;
-  double * w = xf.w + (size_t)(rk * 4 + var) * xf.stride;
-  double * v = xf.v + (size_t)(rk * 4 + var) * xf.stride;
-  const int ne = xf.ne;
-  double vprev = 0.;
-  for (int e = 0; e < n; e++) {
-    const int pe = (e % ne) * 32 + e / ne;   // interleaved position of element e
-    const double l = -pf * ll[e];
-    const double c = 1. - pf * lc[e];
-    const double u = -pf * lu[e];
-    lo[pe] = (e == 0) ? 0. : l;
-    if (e == 0) {
-      w[pe] = 1. / c;
-      vprev = u / c;
-      v[pe] = (n > 1) ? vprev : 0.;
-    } else if (e < n - 1) {
-      const double val = 1. / (c - l * vprev);
-      w[pe] = val;
-      vprev = val * u;
-      v[pe] = vprev;
-    } else {
-      w[pe] = 1. / (c - l * vprev);
-      v[pe] = 0.;
+  const int n = xf.n[var], ne = xf.ne;
+  const double * __restrict__ ll = xf.lap_l[var];
+  const double * __restrict__ lc = xf.lap_c[var];
+  const double * __restrict__ lu = xf.lap_u[var];
+  for (int e = tid; e < n; e += blockDim.x) {
+    sl[e] = e > 0 ? (pf * ll[e]) * (pf * lu[e - 1]) : 0.;
+    sc[e] = 1. - pf * lc[e];
+  }
+  __syncthreads();
+  if (tid == 0) {
+    double t2 = 0., t1 = 1.;   // theta_{e-2}, theta_{e-1}
+    for (int e = 0; e < n; e++) {
+      const double t = sc[e] * t1 - sl[e] * t2;
+      sc[e] = t;
+      su[e] = t1;
+      t2 = t1;
+      t1 = t;
+      const double a = fabs(t1);
+      if (a > 0x1p256) { t1 *= 0x1p-256; t2 *= 0x1p-256; }
+      else if (a < 0x1p-256) { t1 *= 0x1p256; t2 *= 0x1p256; }
     }
+  }
+  __syncthreads();
+  for (int e = tid; e < n; e += blockDim.x) su[e] = su[e] / sc[e];
+  __syncthreads();
+  const size_t row = (size_t)rv * xf.stride;
+  auto fe = [&](int e) { return e > 0 && e < n ? pf * ll[e] * su[e - 1] : 0.; };       // -l_e w_{e-1}
+  auto ge = [&](int e) { return e < n - 1 ? pf * lu[e] * su[e + 1] : 0.; };            // -u_e w_{e+1}
+  for (int e = tid; e < 32 * ne; e += blockDim.x) {
+    const int pe = (e % ne) * 32 + e / ne;   // interleaved position of element e
+    xf.f[row + pe] = fe(e);
+    xf.g[row + pe] = ge(e);
+    xf.w[row + pe] = e < n ? su[e] : 0.;
+  }
+  if (tid < 32) {
+    double pfw = 1., pbw = 1.;   // products over the lane's elements
+    for (int m = 0; m < ne; m++) {
+      pfw *= fe(tid * ne + m);
+      pbw *= ge(tid * ne + m);
+    }
+    double * s = xf.scan + (size_t)rv * XSCAN_ROWS * 32;
+    for (int q = 0; q < 5; q++) {
+      s[q * 32 + tid] = tid >= (1 << q) ? pfw : 0.;
+      s[(5 + q) * 32 + tid] = tid + (1 << q) < 32 ? pbw : 0.;
+      const double a = __shfl_up_sync(0xffffffffu, pfw, 1 << q), b = __shfl_down_sync(0xffffffffu, pbw, 1 << q);
+      pfw = tid >= (1 << q) ? pfw * a : 0.;
+      pbw = tid + (1 << q) < 32 ? pbw * b : 0.;
+    }
+  }
+}
+
+// The rows of FP32-storage contexts: l_e, w_e and v_e = u_e w_e from the division
+// recurrence of gtsv, in its order of roundings (tc_march_f32.cu). The rows are
+// staged in shared memory by the block, so that only the recurrence is serial.
+__global__ void __launch_bounds__(256) xfactor32_kernel(XFactors xf, const double * __restrict__ dtp, double nu, double kappa) {
+  __shared__ double sl[XF_MAX], sc[XF_MAX], su[XF_MAX];   // l; c, then w; u, then v
+  const int rv = blockIdx.x, rk = rv / 4, var = rv % 4, tid = threadIdx.x;
+  const double dt = *dtp;
+  const double diff = (var == VT) ? kappa : nu;
+  double pf = 0.5 * rk_gamma(rk) * dt * diff;
+  if (var == VUX) pf = 2. * pf;
+  const int n = xf.n[var], ne = xf.ne;
+  for (int e = tid; e < n; e += blockDim.x) {
+    sl[e] = -pf * xf.lap_l[var][e];
+    sc[e] = fma(-pf, xf.lap_c[var][e], 1.);
+    su[e] = -pf * xf.lap_u[var][e];
+  }
+  __syncthreads();
+  if (tid == 0) {
+    double vprev = su[0] / sc[0];
+    sc[0] = 1. / sc[0];
+    su[0] = n > 1 ? vprev : 0.;
+    for (int e = 1; e < n; e++) {
+      const double val = 1. / fma(-sl[e], vprev, sc[e]);
+      sc[e] = val;
+      vprev = val * su[e];
+      su[e] = e < n - 1 ? vprev : 0.;
+    }
+  }
+  __syncthreads();
+  const size_t row = (size_t)rv * xf.stride;
+  for (int e = tid; e < n; e += blockDim.x) {
+    const int pe = (e % ne) * 32 + e / ne;
+    xf.f[row + pe] = e > 0 ? sl[e] : 0.;
+    xf.w[row + pe] = sc[e];
+    xf.g[row + pe] = su[e];
   }
 }
 
@@ -435,14 +497,23 @@ void launch_yzfactors(const Geo & g, const YZFactors & yf, const double * dtp, d
 }
 
 // ------------------------------------------------------------ launchers
-int predict_warps(int nx) {
+int predict_warps32(int nx) {
   int w = 1;
   while (32 * w < nx) w *= 2;
   return w;
 }
 
+// warps of the predict kernel per radial line: the instances of tc_march_inst.cuh,
+// powers of two for lines longer than 256 points (the line kernel's elements per lane)
+int predict_warps(int nx) {
+  for (int w : {1, 2, 3, 4, 6, 8, 16})
+    if (32 * w >= nx) return w;
+  return 32;
+}
+
 void launch_xfactors(const XFactors & xf, const double * dtp, double nu, double kappa, cudaStream_t st) {
-  xfactor_kernel<<<1, 32, 0, st>>>(xf, dtp, nu, kappa);
+  if (xf.single) xfactor32_kernel<<<12, 256, 0, st>>>(xf, dtp, nu, kappa);
+  else xfactor_kernel<<<12, 256, 0, st>>>(xf, dtp, nu, kappa);
 }
 
 void launch_apply(const Geo & g, const Bc & bc, const FieldBufs & in, const FieldBufs & out, const DeltaSet & ds,
