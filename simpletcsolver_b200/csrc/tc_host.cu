@@ -530,14 +530,21 @@ static int build_tables(Ctx & c, const domain_t * d) {
   const size_t nspec = (size_t)nx * nz * nyh;
   c.ps.spec_bytes = 2 * c.sb;
   c.ps.spec = valloc(c, nspec * c.ps.spec_bytes);
-  c.ps.vscr = dalloc(c, nspec);
-  if (!c.ps.tw_y || !c.ps.tw_z || !c.ps.spec || !c.ps.vscr) return fail("cudaMalloc of Poisson buffers failed");
-  // radial solves by warps when nx = 32 E: per-line factors computed once
-  c.ps.fe = (nx == 64 || nx == 128 || nx == 256) ? nx / 32 : 0;
+  if (!c.ps.tw_y || !c.ps.tw_z || !c.ps.spec) return fail("cudaMalloc of Poisson buffers failed");
+  // radial solves by warps: per-line factors computed once (rows padded to whole
+  // lanes); without the memory for them, the per-column solves' scratch
+  c.ps.fe = tdm_lines_elements(nx, c.sb == 4);
   if (c.ps.fe) {
-    c.ps.fw = dalloc(c, nspec);
-    c.ps.fv = c.ps.vscr;   // not otherwise used on this path
-    if (!c.ps.fw) return fail("cudaMalloc of Poisson buffers failed");
+    c.ps.fw = dalloc(c, (size_t)nz * nyh * 32 * c.ps.fe);
+    if (!c.ps.fw) {
+      cudaGetLastError();
+      c.ps.fe = 0;
+    }
+  }
+  if (c.ps.fe == 0) {
+    c.ps.vscr = dalloc(c, nspec);
+    if (!c.ps.vscr) return fail("cudaMalloc of Poisson buffers failed");
+  } else {
     launch_tdm_factors(c.g, c.ps, c.tab_y, c.tab_z, c.base, c.st);
     CK(cudaGetLastError());
   }
@@ -560,6 +567,21 @@ static int check_domain(const domain_t * d) {
   if (!d->hxxf || !d->hxxc || !d->hyxf || !d->hyxc || !d->jdxf || !d->jdxc)
     return fail("domain metric arrays are not initialised");
   return 0;
+}
+
+// the kernels' shared-memory limits, once per device (attributes of the kernels,
+// not of a context)
+static void allow_smem() {
+  static std::mutex m;
+  static std::vector<int> done;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  std::lock_guard<std::mutex> lk(m);
+  if (std::find(done.begin(), done.end(), dev) != done.end()) return;
+  poisson_smem_limits();
+  march_smem_limits();
+  allow_periodic_lines_smem();
+  done.push_back(dev);
 }
 
 static Ctx * create_ctx(const domain_t * d, const fluid_t * fl) {
@@ -637,9 +659,7 @@ static Ctx * create_ctx(const domain_t * d, const fluid_t * fl) {
   if (cudaMallocHost(&c->h_scalar, 64 * sizeof(double)) != cudaSuccess) return bad("cudaMallocHost failed");
   if (cudaMallocHost(&c->h_status, sizeof(unsigned) * 4) != cudaSuccess) return bad("cudaMallocHost failed");
   if (build_tables(*c, d)) { destroy_ctx(c); return nullptr; }
-  poisson_smem_limits();
-  march_smem_limits();
-  allow_periodic_lines_smem();
+  allow_smem();
   c->nu = 0.;
   if (set_physics(*c, fl, d)) { destroy_ctx(c); return nullptr; }
   return c;

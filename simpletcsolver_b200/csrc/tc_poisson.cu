@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "tc_common.cuh"
+#include "tc_fft_mixed.cuh"
 #include "tc_kernels.h"
 
 // resident CTAs per SM requested from the register allocator (measured best
@@ -660,8 +661,9 @@ tdm_kernel(Geo g, Poisson ps, const double * __restrict__ tab_y, const double * 
 // Factors of line l = kz nyh + m (the forward elimination of src/tdm.c:24-44
 // with the Neumann ends folded into the diagonal, as in tdm_kernel): the
 // forward sweep y_i = w_i (q_i - l_i y_{i-1}), y_{-1} = 0, and the back
-// substitution x_i = y_i - v_i x_{i+1}, x_n = 0 (v_{n-1} = 0). The pinned mode
-// (line 0) has w_{n-1} = 0, which sets its last unknown to zero.
+// substitution x_i = y_i - v_i x_{i+1}, x_n = 0, with v_i = w_i u_i (formed where
+// it is used; v_{n-1} = 0). The pinned mode (line 0) has w_{n-1} = 0, which sets
+// its last unknown to zero. Rows hold 32 fe values, zero from n on.
 __global__ void tdm_factor_kernel(Geo g, Poisson ps, const double * __restrict__ tab_y,
                                   const double * __restrict__ tab_z, const double * __restrict__ base) {
   const int nyh = ps.nyh, nz = g.nz, n = g.nx, fe = ps.fe;
@@ -675,22 +677,18 @@ __global__ void tdm_factor_kernel(Geo g, Poisson ps, const double * __restrict__
     if (i == n - 1) c += ps.tu[n - 1];
     return c;
   };
-  double * w = ps.fw + (size_t)l * n;
-  double * v = ps.fv + (size_t)l * n;
+  double * w = ps.fw + (size_t)l * 32 * fe;
   auto at = [&](int i) { return (i % fe) * 32 + i / fe; };
   const double c0 = cdiag(0);
   double vprev = ps.tu[0] / c0;
   w[at(0)] = 1. / c0;
-  v[at(0)] = vprev;
   for (int i = 1; i < n - 1; i++) {
     const double val = 1. / (cdiag(i) - ps.tl[i] * vprev);
     vprev = val * ps.tu[i];
     w[at(i)] = val;
-    v[at(i)] = vprev;
   }
   const double last = cdiag(n - 1) - ps.tl[n - 1] * vprev;
   w[at(n - 1)] = (l == 0) ? 0. : 1. / last;
-  v[at(n - 1)] = 0.;
 }
 
 void launch_tdm_factors(const Geo & g, const Poisson & ps, const double * tab_y, const double * tab_z,
@@ -699,86 +697,78 @@ void launch_tdm_factors(const Geo & g, const Poisson & ps, const double * tab_y,
   tdm_factor_kernel<<<(unsigned)((nl + 127) / 128), 128, 0, st>>>(g, ps, tab_y, tab_z, base);
 }
 
-// The radial systems of 16 consecutive lines (kz, m) as one tile: for every i
-// their 16 complex values are contiguous (256 bytes), loaded and stored once;
-// each warp solves whole lines from shared memory with the affine-map scans
-// (E = n / 32 points per lane, in-register prefix + 5-level shuffle scan).
-constexpr int TDM_PT = 16;
-// resident CTAs per SM requested from the register allocator (0: the
-// allocator's own choice), and the factor rows loaded ahead of their use: the
-// warp's first w row with the tile, each line's v row before its forward scan.
-// Measured at 256 x 1024 x 512 (ms per launch): 0.58, prefetched 0.56; 3
-// resident CTAs (80 registers, 64 bytes spilled) 0.58.
-#ifndef TC_TDM_LINES_MB
-#define TC_TDM_LINES_MB 0
-#endif
-#if TC_TDM_LINES_MB > 0
-#define TC_TDM_LINES_BOUNDS __launch_bounds__(256, TC_TDM_LINES_MB)
-#else
-#define TC_TDM_LINES_BOUNDS __launch_bounds__(256)
-#endif
-#ifndef TC_TDM_LINES_PREFETCH
-#define TC_TDM_LINES_PREFETCH 1
-#endif
+// Elements per lane of the warp solves for lines of n points, 0 where the
+// per-column kernel runs: lines of more than 512 points (a tile would not fit) and,
+// in FP32-storage contexts, every length but 64, 128 and 256 (their results hold to
+// the last stored bit). Per launch, per-column -> warps: 192 x 512 x 256 0.254 ->
+// 0.107 ms, 384 x 256 x 128 0.374 -> 0.074, 96 x 180 x 120 0.076 -> 0.016.
+int tdm_lines_elements(int n, bool single) {
+  if (single) return n == 64 || n == 128 || n == 256 ? n / 32 : 0;
+  for (int e : {1, 2, 3, 4, 6, 8, 12, 16})
+    if (n > 1 && n <= 32 * e) return e;
+  return 0;
+}
 
+// The radial systems of PT consecutive lines (kz, m) as one tile: for every i
+// their complex values are contiguous (256 bytes for 16), loaded and stored once;
+// each warp solves whole lines from shared memory with the affine-map scans
+// (E points per lane, in-register prefix + 5-level shuffle scan). Points from n
+// on map to zero (w = 0).
+// Bound: HBM, 32 bytes a value read and written and 8 of factors; the warp's first
+// w row loads with the tile. Measured at 256 x 1024 x 512 (ms per launch): with the
+// back-substitution factors read from memory too 0.56, formed from w 0.52.
+constexpr int tdm_pt(int E) { return E > 8 ? 8 : 16; }   // lines per tile, at most 65 KB
 template <int E, class Z>
-__global__ void TC_TDM_LINES_BOUNDS tdm_lines_kernel(Geo g, Poisson ps) {
-  constexpr int N = 32 * E, NT = 256, PER = N * TDM_PT / NT;
+__global__ void __launch_bounds__(256) tdm_lines_kernel(Geo g, Poisson ps) {
+  constexpr int N = 32 * E, NT = 256, PT = E > 8 ? 8 : 16, PER = N * PT / NT;
   extern __shared__ double2 tq[];
-  const int nyh = ps.nyh;
+  const int nyh = ps.nyh, n = g.nx;
   const long long nlines = (long long)nyh * g.nz;
-  const long long l0 = (long long)blockIdx.x * TDM_PT;
-  const int nt = (int)min((long long)TDM_PT, nlines - l0);
+  const long long l0 = (long long)blockIdx.x * PT;
+  const int nt = (int)min((long long)PT, nlines - l0);
   const size_t st = (size_t)nlines;               // complex values between radial indices
   Z * spec = static_cast<Z *>(ps.spec);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#if TC_TDM_LINES_PREFETCH
   double wq[E];   // w of the warp's first line, in flight with the tile
   if (wid < nt) {
     const double * w = ps.fw + (size_t)(l0 + wid) * N;
 #pragma unroll
     for (int e = 0; e < E; e++) wq[e] = w[e * 32 + lane];
   }
-#endif
   {
     double2 buf[PER];
 #pragma unroll
     for (int r = 0; r < PER; r++) {
-      const int q = threadIdx.x + r * NT, t = q % TDM_PT, i = q / TDM_PT;
-      buf[r] = t < nt ? zget(spec + (size_t)i * st + l0 + t) : make_double2(0., 0.);
+      const int q = threadIdx.x + r * NT, t = q % PT, i = q / PT;
+      buf[r] = t < nt && i < n ? zget(spec + (size_t)i * st + l0 + t) : make_double2(0., 0.);
     }
 #pragma unroll
     for (int r = 0; r < PER; r++) {
-      const int q = threadIdx.x + r * NT, t = q % TDM_PT, i = q / TDM_PT;
-      tq[i * TDM_PT + (t ^ ((i / E) & (TDM_PT - 1)))] = buf[r];
+      const int q = threadIdx.x + r * NT, t = q % PT, i = q / PT;
+      tq[i * PT + (t ^ ((i / E) & (PT - 1)))] = buf[r];
     }
   }
+  // l_i, and u_i of the back substitution, as the lanes read them (registers for
+  // the two rows cost a resident block at E = 8: 0.79 ms per launch)
+  double * const sl = reinterpret_cast<double *>(tq + N * PT), * const su = sl + N;
+  for (int q = threadIdx.x; q < N; q += NT) {
+    const int i = (q & 31) * E + (q >> 5);
+    sl[q] = i < n ? ps.tl[i] : 0.;
+    su[q] = i < n - 1 ? ps.tu[i] : 0.;
+  }
   __syncthreads();
-  double ll[E];
-#pragma unroll
-  for (int e = 0; e < E; e++) ll[e] = ps.tl[lane * E + e];
   for (int t = wid; t < nt; t += NT / 32) {
     const long long l = l0 + t;
     const double * w = ps.fw + (size_t)l * N;
-    const double * v = ps.fv + (size_t)l * N;
-    const int sw = t ^ (lane & (TDM_PT - 1));
-    double fa[E], bre[E], bim[E];
-#if TC_TDM_LINES_PREFETCH
-    double vq[E];
-#pragma unroll
-    for (int e = 0; e < E; e++) vq[e] = v[e * 32 + lane];
-#endif
+    const int sw = t ^ (lane & (PT - 1));
+    double fa[E], bre[E], bim[E], we[E];
 #pragma unroll
     for (int e = 0; e < E; e++) {
-      const double2 qv = tq[(lane * E + e) * TDM_PT + sw];
-#if TC_TDM_LINES_PREFETCH
-      const double we = (t == wid) ? wq[e] : w[e * 32 + lane];
-#else
-      const double we = w[e * 32 + lane];
-#endif
-      fa[e] = -we * ll[e];
-      bre[e] = we * qv.x;
-      bim[e] = we * qv.y;
+      const double2 qv = tq[(lane * E + e) * PT + sw];
+      we[e] = (t == wid) ? wq[e] : w[e * 32 + lane];
+      fa[e] = -we[e] * sl[e * 32 + lane];
+      bre[e] = we[e] * qv.x;
+      bim[e] = we[e] * qv.y;
     }
     // forward: prefix of the lane's maps, then across lanes
 #pragma unroll
@@ -807,11 +797,7 @@ __global__ void TC_TDM_LINES_BOUNDS tdm_lines_kernel(Geo g, Poisson ps) {
     }
     // backward: x_i = y_i - v_i x_{i+1}, suffix maps
 #pragma unroll
-#if TC_TDM_LINES_PREFETCH
-    for (int e = 0; e < E; e++) fa[e] = -vq[e];
-#else
-    for (int e = 0; e < E; e++) fa[e] = -v[e * 32 + lane];
-#endif
+    for (int e = 0; e < E; e++) fa[e] = -(we[e] * su[e * 32 + lane]);
 #pragma unroll
     for (int d = 1; d < E; d <<= 1) {
 #pragma unroll
@@ -835,25 +821,28 @@ __global__ void TC_TDM_LINES_BOUNDS tdm_lines_kernel(Geo g, Poisson ps) {
     if (lane == 31) { xre = 0.; xim = 0.; }
 #pragma unroll
     for (int e = 0; e < E; e++)
-      tq[(lane * E + e) * TDM_PT + sw] = make_double2(fa[e] * xre + bre[e], fa[e] * xim + bim[e]);
+      tq[(lane * E + e) * PT + sw] = make_double2(fa[e] * xre + bre[e], fa[e] * xim + bim[e]);
   }
   __syncthreads();
 #pragma unroll 8
   for (int r = 0; r < PER; r++) {
-    const int q = threadIdx.x + r * NT, t = q % TDM_PT, i = q / TDM_PT;
-    if (t < nt) zput(spec + (size_t)i * st + l0 + t, tq[i * TDM_PT + (t ^ ((i / E) & (TDM_PT - 1)))]);
+    const int q = threadIdx.x + r * NT, t = q % PT, i = q / PT;
+    if (t < nt && i < n) zput(spec + (size_t)i * st + l0 + t, tq[i * PT + (t ^ ((i / E) & (PT - 1)))]);
   }
 }
 
+// lines per tile: X(E) for every E of tdm_lines_elements
+#define TDM_LINES(X) X(1) X(2) X(3) X(4) X(6) X(8) X(12) X(16)
 template <class Z>
 static bool launch_tdm_lines(const Geo & g, const Poisson & ps, cudaStream_t st) {
   const long long nl = (long long)ps.nyh * g.nz;
-  const unsigned nblk = (unsigned)((nl + TDM_PT - 1) / TDM_PT);
-  const size_t smem = sizeof(double2) * (size_t)g.nx * TDM_PT;
+  const int pt = tdm_pt(ps.fe);
+  const unsigned nblk = (unsigned)((nl + pt - 1) / pt);
+  const size_t smem = sizeof(double2) * (size_t)32 * ps.fe * (pt + 1);
   switch (ps.fe) {
-    case 2: tdm_lines_kernel<2, Z><<<nblk, 256, smem, st>>>(g, ps); return true;
-    case 4: tdm_lines_kernel<4, Z><<<nblk, 256, smem, st>>>(g, ps); return true;
-    case 8: tdm_lines_kernel<8, Z><<<nblk, 256, smem, st>>>(g, ps); return true;
+#define X(E) case E: tdm_lines_kernel<E, Z><<<nblk, 256, smem, st>>>(g, ps); return true;
+    TDM_LINES(X)
+#undef X
     default: return false;
   }
 }
@@ -1019,9 +1008,115 @@ iffty_kernel(Geo g, Poisson ps, int P, int lg, double * __restrict__ psi) {
   }
 }
 
+// --------------------------------------------------------------- mixed radices
+// The transforms of lengths that are not powers of two (FP64 contexts), with the
+// input and output of the power-of-two kernels above; tc_fft_mixed.cuh.
+
+// divergence of a plane's radial indices i0 .. i0 + 2P - 1, then its r2c
+// transforms along y, two real lines per complex one
+__global__ void __launch_bounds__(256) div_mixy_kernel(Geo g, Coefs cf, Poisson ps, Radices rd, int P,
+                                                       const double * __restrict__ ux, const double * __restrict__ uy,
+                                                       const double * __restrict__ uz, const double * __restrict__ dtp,
+                                                       int rkstep) {
+  extern __shared__ double2 smem[];
+  const int ny = g.ny, nx = g.nx, nz = g.nz, nyh = ps.nyh, TI = 2 * P, LS = mixed_len(ny);
+  double2 * const a = smem, * const b = smem + (size_t)P * LS;
+  const int i0 = blockIdx.x * TI + 1, k = blockIdx.y + 1;
+  const double prefactor = 1. / (rk_gamma(rkstep) * (*dtp)) / (1. * ny * nz);
+  // the passes after the first alternate a -> b -> a; the divergence goes where the first pass does not write
+  for (int idx = threadIdx.x; idx < TI * ny; idx += blockDim.x) {
+    const int ii = idx & (TI - 1), j = idx / TI + 1, i = i0 + ii;
+    double val = 0.;
+    if (i <= nx) {
+      const size_t f = fidx(g, i, j, k), c = cidx(g, i, j, k);
+      const double jy = __ldg(cf.c_e1 + i), jz = __ldg(cf.c_e2 + i);
+      val = prefactor * (__ldg(cf.c_invjdxc + i) *
+                         (-__ldg(cf.c_jf + i) * __ldg(ux + f) + __ldg(cf.c_jf + i + 1) * __ldg(ux + f + 1) -
+                          jy * __ldg(uy + c) + jy * __ldg(uy + c + nx + 2) - jz * __ldg(uz + c) +
+                          jz * __ldg(uz + c + (size_t)(nx + 2) * (ny + 2))));
+    }
+    reinterpret_cast<double *>(b + (ii >> 1) * LS)[2 * mpad(j - 1) + (ii & 1)] = val;
+  }
+  __syncthreads();
+  double2 * const z = (rd.count & 1) ? a : b;   // where the last pass leaves the lines
+  mixed_fft<-1, false>(rd, ny, P, a, b, LS, ps.tw_y, [&](int p, int e) { return b[p * LS + mpad(e)]; },
+                       [&](int p, int e, double2 v) { z[p * LS + mpad(e)] = v; });
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < TI * nyh; idx += blockDim.x) {
+    const int ii = idx / nyh, m = idx - ii * nyh, i = i0 + ii;
+    if (i > nx) continue;
+    const double2 zm = z[(ii >> 1) * LS + mpad(m)], zn = z[(ii >> 1) * LS + mpad(m == 0 ? 0 : ny - m)];
+    double2 out;
+    if ((ii & 1) == 0) out = make_double2(0.5 * (zm.x + zn.x), 0.5 * (zm.y - zn.y));
+    else out = make_double2(0.5 * (zm.y + zn.y), -0.5 * (zm.x - zn.x));
+    static_cast<double2 *>(ps.spec)[((size_t)(i - 1) * nz + (k - 1)) * nyh + m] = out;
+  }
+}
+
+// transforms along z of wavenumbers m0 .. m0 + P - 1 of one radial index, in place
+template <int SIGN>
+__global__ void __launch_bounds__(256) mixz_kernel(Geo g, Poisson ps, Radices rd, int P) {
+  extern __shared__ double2 smem[];
+  const int nz = g.nz, nyh = ps.nyh, LS = mixed_len(nz), m0 = blockIdx.x * P;
+  double2 * const col = static_cast<double2 *>(ps.spec) + (size_t)blockIdx.y * nz * nyh + m0;
+  mixed_fft<SIGN, true>(rd, nz, P, smem, smem + (size_t)P * LS, LS, ps.tw_z,
+                        [&](int p, int e) { return m0 + p < nyh ? col[(size_t)e * nyh + p] : make_double2(0., 0.); },
+                        [&](int p, int e, double2 v) { if (m0 + p < nyh) col[(size_t)e * nyh + p] = v; });
+}
+
+// c2r transforms along y into psi with its Neumann x ghosts and periodic images
+__global__ void __launch_bounds__(256) imixy_kernel(Geo g, Poisson ps, Radices rd, int P, double * __restrict__ psi) {
+  extern __shared__ double2 smem[];
+  const int ny = g.ny, nx = g.nx, nz = g.nz, nyh = ps.nyh, half = ny >> 1, TI = 2 * P, LS = mixed_len(ny);
+  double2 * const a = smem, * const b = smem + (size_t)P * LS;
+  const int i0 = blockIdx.x * TI + 1, k = blockIdx.y + 1;
+  const double2 * sp = static_cast<const double2 *>(ps.spec);
+  // Hermitian extension of the two packed real lines (DC and Nyquist: real parts)
+  for (int idx = threadIdx.x; idx < P * nyh; idx += blockDim.x) {
+    const int pp = idx / nyh, m = idx - pp * nyh, ia = i0 + 2 * pp;
+    double2 xa = make_double2(0., 0.), xb = xa;
+    if (ia <= nx) xa = sp[((size_t)(ia - 1) * nz + (k - 1)) * nyh + m];
+    if (ia + 1 <= nx) xb = sp[((size_t)ia * nz + (k - 1)) * nyh + m];
+    double2 * line = b + pp * LS;
+    if (m == 0 || m == half) {
+      line[mpad(m)] = make_double2(xa.x, xb.x);
+    } else {
+      line[mpad(m)] = make_double2(xa.x - xb.y, xa.y + xb.x);
+      line[mpad(ny - m)] = make_double2(xa.x + xb.y, -xa.y + xb.x);
+    }
+  }
+  __syncthreads();
+  double2 * const z = (rd.count & 1) ? a : b;
+  mixed_fft<+1, false>(rd, ny, P, a, b, LS, ps.tw_y, [&](int p, int e) { return b[p * LS + mpad(e)]; },
+                       [&](int p, int e, double2 v) { z[p * LS + mpad(e)] = v; });
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < TI * ny; idx += blockDim.x) {
+    const int ii = idx & (TI - 1), j = idx / TI + 1, i = i0 + ii;
+    if (i > nx) continue;
+    const double2 v = z[(ii >> 1) * LS + mpad(j - 1)];
+    const double val = (ii & 1) ? v.y : v.x;
+    auto put = [&](int jj, int kk) {
+      const size_t q = cidx(g, i, jj, kk);
+      psi[q] = val;
+      if (i == 1) psi[q - 1] = val;
+      if (i == nx) psi[q + 1] = val;
+    };
+    put(j, k);
+    for_images(j, k, ny, nz, put);
+  }
+}
+
+// lines per block of the mixed transforms: a power of two, about 2048 points and
+// at most 56 KB of shared memory for both copies (a longest line alone: 70 KB)
+static int mixed_lines(int n, int cap) {
+  int p = 64;
+  while (p > 1 && (p * n > 3072 || 2 * sizeof(double2) * p * mixed_len(n) > 56 * 1024 || p / 2 >= cap)) p >>= 1;
+  return p;
+}
+
 // --------------------------------------------------------------- direct DFTs
-// Lengths that are not powers of two (even ny, nz a multiple of 4, as FFTW
-// plans any length: compute_potential.c:247-309) take direct transforms: each
+// FP32-storage contexts take direct transforms for lengths that are not powers of
+// two (their results hold to the last stored bit; tc_march_f32.cu): each
 // output wavenumber is the sum over the line with twiddles tw[(j m) mod N] =
 // exp(-2 pi i (j m mod N) / N) from the same tables. O(N^2) per line, FP64
 // accumulation, FFTW's conventions (unnormalised, r2c keeps N/2+1 terms, c2r
@@ -1151,7 +1246,15 @@ static void launch_poisson_t(const Geo & g, const Coefs & cf, const Poisson & ps
   const size_t smy = sizeof(Z) * (size_t)Py * padded_len(g.ny);
   dim3 gy((g.nx + 2 * Py - 1) / (2 * Py), g.nz);
   const dim3 gl(g.nx, g.nz);   // one CTA per (i, k) line of the direct transforms in y
+  constexpr bool MIX = sizeof(Z) == 16;   // FP64 contexts: mixed radices; FP32-storage ones: direct sums
+  const int My = mixed_lines(g.ny, (g.nx + 1) / 2), Mz = mixed_lines(g.nz, ps.nyh);
+  const dim3 gmy((g.nx + 2 * My - 1) / (2 * My), g.nz), gmz((ps.nyh + Mz - 1) / Mz, g.nx);
+  const size_t smmy = 2 * sizeof(double2) * (size_t)My * mixed_len(g.ny);
+  const size_t smmz = 2 * sizeof(double2) * (size_t)Mz * mixed_len(g.nz);
+  const Radices ry = radices_of(g.ny), rz = radices_of(g.nz);
   if (fy) div_ffty_kernel<EPTY, T, Z><<<gy, Py * tply, smy, st>>>(g, cf, ps, Py, lgy, f.ux, f.uy, f.uz, dtp, rkstep);
+  else if constexpr (MIX)
+    div_mixy_kernel<<<gmy, 256, smmy, st>>>(g, cf, ps, ry, My, f.ux, f.uy, f.uz, dtp, rkstep);
   else div_dfty_kernel<T, Z><<<gl, 128, sizeof(double) * g.ny, st>>>(g, cf, ps, f.ux, f.uy, f.uz, dtp, rkstep);
   mark(pm.k_div);
   const int Pz = lines_per_cta(g.nz, ps.nyh, EPTZ, TC_FFTZ_THREADS);
@@ -1164,6 +1267,7 @@ static void launch_poisson_t(const Geo & g, const Coefs & cf, const Poisson & ps
 #endif
   const dim3 gc(ps.nyh, g.nx);   // one CTA per (ky, i) column of the direct transforms in z
   if (fz) fftz_kernel<EPTZ, -1, Z><<<gz, Pz * tplz, smz, st>>>(g, ps, Pz, lgz);
+  else if constexpr (MIX) mixz_kernel<-1><<<gmz, 256, smmz, st>>>(g, ps, rz, Mz);
   else dftz_kernel<-1, Z><<<gc, 128, sizeof(double2) * g.nz, st>>>(g, ps);
   mark(pm.k_fwd);
   if (!launch_tdm_lines<Z>(g, ps, st)) {
@@ -1172,6 +1276,7 @@ static void launch_poisson_t(const Geo & g, const Coefs & cf, const Poisson & ps
   }
   mark(pm.k_tdm);
   if (fz) fftz_kernel<EPTZ, +1, Z><<<gz, Pz * tplz, smz, st>>>(g, ps, Pz, lgz);
+  else if constexpr (MIX) mixz_kernel<+1><<<gmz, 256, smmz, st>>>(g, ps, rz, Mz);
   else dftz_kernel<+1, Z><<<gc, 128, sizeof(double2) * g.nz, st>>>(g, ps);
   mark(pm.k_inv);
   constexpr bool bulk = sizeof(Z) == 16;   // staged spectrum rows need 16-byte values
@@ -1179,6 +1284,7 @@ static void launch_poisson_t(const Geo & g, const Coefs & cf, const Poisson & ps
     iffty_kernel<EPTY, Z, bulk><<<gy, Py * tply, smy + 16, st>>>(g, ps, Py, lgy, f.psi);
   else if (fy)
     iffty_kernel<EPTY, Z, false><<<gy, Py * tply, smy, st>>>(g, ps, Py, lgy, f.psi);
+  else if constexpr (MIX) imixy_kernel<<<gmy, 256, smmy, st>>>(g, ps, ry, My, f.psi);
   else idfty_kernel<Z><<<gl, 128, sizeof(double2) * ps.nyh, st>>>(g, ps, f.psi);
   mark(pm.k_ify);
 }
@@ -1241,9 +1347,14 @@ static void poisson_smem_limits_s() {
 void poisson_smem_limits() {
   poisson_smem_limits_s<double, double2>();
   poisson_smem_limits_s<float, float2>();
-  allow_dyn_smem(tdm_lines_kernel<8, double2>);
+  allow_dyn_smem(div_mixy_kernel);
+  allow_dyn_smem(imixy_kernel);
+  allow_dyn_smem(mixz_kernel<-1>);
+  allow_dyn_smem(mixz_kernel<+1>);
+#define X(E) allow_dyn_smem(tdm_lines_kernel<E, double2>);
+  TDM_LINES(X)
+#undef X
   allow_dyn_smem(tdm_lines_kernel<8, float2>);
-  allow_dyn_smem(tdm_lines_kernel<4, double2>);
   allow_dyn_smem(tdm_lines_kernel<4, float2>);
 }
 

@@ -10,7 +10,7 @@ import pytest
 
 from oracle import tc_numpy as tn
 from simpletcsolver_b200 import abi, ic
-from simpletcsolver_b200.solver import Solver, params_of
+from simpletcsolver_b200.solver import Solver
 
 pytestmark = pytest.mark.gpu
 
@@ -23,8 +23,7 @@ SHAPES = [
 
 
 def run_oracle(case, d0):
-    prm = params_of(case)
-    prm = tn.Params(prm.uy_xm, prm.uy_xp, prm.t_xm, prm.t_xp, case.implicit, case.coef_dt_adv, case.coef_dt_dif)
+    prm = tn.Params(case.uy_xm, case.uy_xp, case.t_xm, case.t_xp, case.implicit, case.coef_dt_adv, case.coef_dt_dif)
     d = tn.load_domain(d0)
     fl = tn.load_fluid(d, d0, case.Re, case.Pr, prm)
     dt = tn.decide_dt(d, fl, prm)
