@@ -164,7 +164,6 @@ __device__ __forceinline__ float gelu_grad(float z) {
 // ---- convolution: forward and input gradient ------------------------------
 constexpr int TX = 8, TY = 16;             // output tile: 8 x, 16 y, one z plane (M = 128)
 constexpr int HX = TX + 2, HY = TY + 2;    // halo of one plane
-constexpr int NN_THREADS = 128;            // weight gradient: 4 warps, one TMEM lane quarter each
 // epilogue warps: groups of four (one per TMEM lane quarter), each group
 // draining every NGRP-th output plane; halo loader warps
 #ifndef TC_CONV_EPI_GROUPS
@@ -550,210 +549,323 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) conv3_kernel(ConvArgs A) {
 // D (M = 128, N = COUT) += A (M x K = 16 cells) B^T, both operands MN-major:
 // A is the input halo (a 16-byte unit = 8 channels of one cell; channel chunks
 // at CHB continue into the next halo row, so rows m = (y shift s, ci) cover
-// NSH = 128 / CIN shifts s = dy + 1 of one (dz, dx) pair); B is the gradient
-// tile of the plane, units [y][co chunk][x]. Nine accumulators (dz, dx) of
-// COUT columns each live in tensor memory for the whole life of the CTA,
-// which loops over (column tile, z chunk) work items; the CTA writes its raw
-// partial sums, reduced afterwards by wgrad_reduce_kernel.
+// NSH = 128 / CIN shifts s = dy + 1 of one dx); B is the gradient tiles of the
+// three planes z = p - 1, p, p + 1 that input plane p meets (taps dz = p - z = 1,
+// 0, -1), side by side along N, so one MMA serves three taps. The tiles lie in a
+// ring of NG plane slots interleaved per row, units [y][slot][co chunk][x], whose
+// first two slots are kept twice (NG, NG + 1), so a window of three never wraps.
+// Three accumulators (dx) of 3 COUT columns live in tensor memory for the whole
+// life of the CTA, zeroed first, so every MMA accumulates. A CTA takes an equal
+// contiguous share of the planes of all column tiles (ConvCursor) and writes its
+// raw partial sums, reduced afterwards by wgrad_reduce_kernel.
+//
+// Roles, meeting at mbarriers only: loader warps bring halo plane p and gradient
+// tile p + 1 of each step; one thread of the MMA warp issues a step's 24 MMAs,
+// whose commit releases the halo slot and the tile of p - 1; the readout warps sum
+// each tile for the bias gradient meanwhile and drain the accumulators at the end.
+// Bound: the MMAs (an M = 128, K = 16 MMA takes about 62 cycles at N = 32, 72 of
+// them a plane 4.5 k cycles; 24 at N = 96 well under 2 k) and the copies. A 32 -> 32 layer
+// of 64 x 256 x 128 cells: 0.59 ms with one role, two block barriers and a serial
+// bias sum per plane; 0.37 with roles and N = 32; 0.20 now.
+constexpr int WG_LOADERS = 4, WG_MMA = 4;             // readout warps 0 .. 3, the MMA warp, the loaders
+constexpr int WG_THREADS = 32 * (WG_MMA + 1 + WG_LOADERS);
 template <int CIN, int COUT>
 struct WgradLayout {
   static constexpr int NSH = 128 / CIN;                  // y shifts per accumulator
   static constexpr int HYW = TY + NSH - 1;               // halo rows y0 - 1 .. y0 + TY + NSH - 3
   static constexpr int CHB = HX * 16;
   static constexpr int ROWB = (CIN / 8) * CHB;
-  static constexpr int SLOTB = HYW * ROWB;
-  static constexpr int GB = TY * (COUT / 8) * TX * 16;   // gradient tile of one plane
-  static constexpr int NSW = 5, NGS = 3;                 // halo and gradient slots: MMAs of two planes in flight
-  static constexpr int GOFF = NSW * SLOTB;               // gradient slots after the halo ring
-  static constexpr int BAR = GOFF + NGS * GB;            // two mbarriers, then the TMEM address
-  static constexpr int USED = BAR + 32;
+  static constexpr int HB = HYW * ROWB;                  // a halo plane
+  static constexpr int NSW = 6;                          // halo slots
+  static constexpr int LAG = 3;                          // planes between a plane's copies and its announcement
+  static constexpr int NG = 7;                           // gradient slots in the ring (three in use)
+  static constexpr int GP = (COUT / 8) * TX * 16;        // one row of a gradient tile
+  static constexpr int GROW = (NG + 2) * GP;             // a row of all slots
+  static constexpr int GOFF = NSW * HB;
+  static constexpr int BAR = GOFF + TY * GROW;           // full[NSW], free[NSW], gfree[NG], done, TMEM address, abort flag
+  static constexpr int NBAR = 2 * NSW + NG + 1;
+  static constexpr int RED = BAR + NBAR * 8 + 16;        // [4][COUT] floats: the readout warps' bias sums
+  static constexpr int USED = RED + 4 * COUT * 4;
   static constexpr int TCOLS = 9 * COUT > 256 ? 512 : 256;
   // one CTA per SM, so that its tensor-memory allocation never waits on
   // another CTA's: ask for more than half of the shared memory
   static constexpr int BYTES = USED < 120 * 1024 ? 120 * 1024 : USED;
+  static_assert(HB % 16 == 0 && BAR % 16 == 0 && BYTES <= 227 * 1024, "shared memory");
 };
 
 struct WgradArgs {
-  int nx, ny, nz, zc, nitems;
+  int nx, ny, nz;
   const __nv_bfloat16 * x;    // [cell][CIN] layer input
   const __nv_bfloat16 * dy;   // [cell][COUT] gradient of the layer's pre-activation
   float * part;               // [gridDim.x][9][128][COUT] raw sums, then [gridDim.x][COUT] bias sums
   unsigned * status;
 };
 
-template <int CIN>
-__device__ __forceinline__ void load_halo_w(char * slot, const __nv_bfloat16 * in, int nx, int ny, int x0, int y0,
-                                            int kp, int hyw) {
+// a loader thread's share of one halo plane (global plane kp)
+template <int CIN, int COUT>
+__device__ __forceinline__ void load_wgrad_halo(char * slot, const WgradArgs & A, int x0, int y0, int kp, int lt) {
+  using L = WgradLayout<CIN, COUT>;
   constexpr int CC = CIN / 8;
-  for (int u = threadIdx.x; u < hyw * HX * CC; u += NN_THREADS) {
+  for (int u = lt; u < L::HYW * HX * CC; u += 32 * WG_LOADERS) {
     const int cc = u % CC, xh = (u / CC) % HX, yh = u / (CC * HX);
     const int i = x0 - 1 + xh;
-    int j = (y0 - 1 + yh) % ny;
-    if (j < 0) j += ny;
-    const bool valid = i >= 0 && i < nx;
-    const __nv_bfloat16 * src = in + ((size_t)((size_t)kp * ny + j) * nx + (valid ? i : 0)) * CIN + cc * 8;
+    int j = y0 - 1 + yh;
+    if (j >= A.ny) j -= A.ny;   // at most NSH - 2 rows past the tile, ny >= 16
+    if (j < 0) j += A.ny;
+    const bool valid = i >= 0 && i < A.nx;
+    const __nv_bfloat16 * src = A.x + ((size_t)((size_t)kp * A.ny + j) * A.nx + (valid ? i : 0)) * CIN + cc * 8;
     cp16(slot + ((yh * CC + cc) * HX + xh) * 16, src, valid);
   }
 }
-template <int COUT>
-__device__ __forceinline__ void load_grad_tile(char * slot, const __nv_bfloat16 * dy, int nx, int ny, int x0, int y0,
-                                               int z) {
-  constexpr int CC = COUT / 8;
-  for (int u = threadIdx.x; u < TY * TX * CC; u += NN_THREADS) {
-    const int cc = u % CC, x = (u / CC) % TX, y = u / (CC * TX);
-    const __nv_bfloat16 * src = dy + ((size_t)((size_t)z * ny + y0 + y) * nx + x0 + x) * COUT + cc * 8;
-    cp16(slot + ((y * CC + cc) * TX + x) * 16, src, true);
+// and of the gradient tile of plane z, into ring slot g (and its second copy)
+template <int CIN, int COUT>
+__device__ __forceinline__ void load_wgrad_tile(char * tiles, const WgradArgs & A, int x0, int y0, int z, int g, int lt) {
+  using L = WgradLayout<CIN, COUT>;
+  constexpr int CG = COUT / 8;
+  for (int u = lt; u < TY * TX * CG; u += 32 * WG_LOADERS) {
+    const int cc = u % CG, x = (u / CG) % TX, y = u / (CG * TX);
+    const __nv_bfloat16 * src = A.dy + ((size_t)((size_t)z * A.ny + y0 + y) * A.nx + x0 + x) * COUT + cc * 8;
+    char * d = tiles + y * L::GROW + g * L::GP + (cc * TX + x) * 16;
+    cp16(d, src, true);
+    if (g < 2) cp16(d + L::NG * L::GP, src, true);
   }
 }
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(NN_THREADS, 1) conv3_wgrad_kernel(WgradArgs A) {
+__global__ void __launch_bounds__(WG_THREADS, 1) conv3_wgrad_kernel(WgradArgs A) {
   using L = WgradLayout<CIN, COUT>;
+  constexpr int NS = L::NSW, NG = L::NG, CG = COUT / 8;
   extern __shared__ __align__(128) char smw[];
-  char * halo = smw;
-  char * gsl = smw + L::GOFF;
-  unsigned long long * bar = reinterpret_cast<unsigned long long *>(smw + L::BAR);   // two
-  unsigned * tslot = reinterpret_cast<unsigned *>(smw + L::BAR + 16);
+  char * tiles = smw + L::GOFF;
+  unsigned long long * full = reinterpret_cast<unsigned long long *>(smw + L::BAR);
+  unsigned long long * sfree = full + NS;
+  unsigned long long * gfree = sfree + NS;
+  unsigned long long * fin = gfree + NG;
+  unsigned * tslot = reinterpret_cast<unsigned *>(fin + 1);
+  volatile int * abort_flag = reinterpret_cast<volatile int *>(tslot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nbx = A.nx / TX, ncol = nbx * (A.ny / TY);
-
-  if (warp == 0) tmem_alloc(tslot, L::TCOLS);
+  if (warp == WG_MMA) tmem_alloc(tslot, L::TCOLS);
   if (tid == 0) {
-    nn_mbar_init(&bar[0], 1);
-    nn_mbar_init(&bar[1], 1);
+    for (int s = 0; s < NS; s++) {
+      nn_mbar_init(&full[s], 32 * WG_LOADERS);
+      nn_mbar_init(&sfree[s], 1 + 4);   // the MMAs' commit and the readout warps, which keep within NS steps
+    }
+    for (int g = 0; g < NG; g++) nn_mbar_init(&gfree[g], 1 + 4);   // the MMAs' commit and the readout warps
+    nn_mbar_init(fin, 1);
+    *abort_flag = 0;
     fence_barrier_init();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = *tslot;
-  constexpr uint32_t IDESC = instr_desc_bf16(128, COUT, 1, 1);
-  float bsum = 0.f;                 // bias gradient of channel tid (tid < COUT)
-  bool first = true;                // no accumulator written yet
-  unsigned phase[2] = {0u, 0u};
-  int pending[2] = {0, 0};          // commits on each barrier not yet waited for
-  bool bad = false;
-  // wait for the MMAs committed on barrier b (bounded)
-  auto drain = [&](int b) {
-    if (!pending[b]) return;
-    const bool ok = nn_mbar_wait(&bar[b], phase[b]);
-    phase[b] ^= 1u;
-    pending[b] = 0;
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) atomicOr(A.status, ST_TIMEOUT);
-      bad = true;
-    }
-  };
-
-  // Per plane z: (a) the MMAs of plane z - 2 have finished (their barrier is
-  // the one plane z commits on), so the halo slot of z + 2 and the gradient
-  // slot of z + 1 are free; (b) issue those copies; (c) wait for the planes up
-  // to z + 1 and the tile of z; (d) issue the plane's 72 MMAs; the MMAs of
-  // z - 1 and z overlap the copies of the next planes.
-  for (int item = blockIdx.x; item < A.nitems && !bad; item += gridDim.x) {
-    const int col = item % ncol, zch = item / ncol;
-    const int x0 = (col % nbx) * TX, y0 = (col / nbx) * TY;
-    const int z0 = zch * A.zc, z1 = min(z0 + A.zc, A.nz);
-    drain(0);
-    drain(1);
-    if (bad) break;
-    load_halo_w<CIN>(halo + 0 * L::SLOTB, A.x, A.nx, A.ny, x0, y0, wrapi(z0 - 1, A.nz), L::HYW);
-    load_halo_w<CIN>(halo + 1 * L::SLOTB, A.x, A.nx, A.ny, x0, y0, z0, L::HYW);
-    load_halo_w<CIN>(halo + 2 * L::SLOTB, A.x, A.nx, A.ny, x0, y0, wrapi(z0 + 1, A.nz), L::HYW);
-    load_grad_tile<COUT>(gsl + 1 * L::GB, A.dy, A.nx, A.ny, x0, y0, z0);   // tile of plane z in slot r % 3
-    cp_commit();
-    for (int z = z0, it = 0; z < z1; z++, it++) {
-      const int r = z - z0 + 1;
-      drain(it & 1);
-      if (bad) break;
-      if (z + 2 <= z1) load_halo_w<CIN>(halo + ((r + 2) % L::NSW) * L::SLOTB, A.x, A.nx, A.ny, x0, y0,
-                                        wrapi(z + 2, A.nz), L::HYW);
-      if (z + 1 < z1) load_grad_tile<COUT>(gsl + ((r + 1) % L::NGS) * L::GB, A.dy, A.nx, A.ny, x0, y0, z + 1);
-      cp_commit();
-      cp_wait<1>();
-      fence_proxy_async();
-      __syncthreads();
-      const char * g = gsl + (r % L::NGS) * L::GB;
-      if (tid == 0) {
-        tc_fence_after();
-        const unsigned hb = su32(halo), gb = su32(g);
-        const unsigned sb[3] = {hb + ((r - 1) % L::NSW) * L::SLOTB, hb + (r % L::NSW) * L::SLOTB,
-                                hb + ((r + 1) % L::NSW) * L::SLOTB};
-#pragma unroll
-        for (int a = 0; a < 9; a++) {
-          const int dz = a / 3 - 1, dx = a % 3 - 1;
-          const unsigned a0 = sb[dz + 1] + (1 + dx) * 16;
-#pragma unroll
-          for (int s = 0; s < TY / 2; s++) {
-            const uint64_t ad = smem_desc(a0 + 2 * s * L::ROWB, L::ROWB, L::CHB);
-            const uint64_t bd = smem_desc(gb + 2 * s * (COUT / 8) * TX * 16, (COUT / 8) * TX * 16, TX * 16);
-            mma_bf16(tmem + a * COUT, ad, bd, IDESC, !(first && s == 0));
-          }
-        }
-        mma_commit(&bar[it & 1]);
-      }
-      pending[it & 1] = 1;
-      if (tid < COUT) {   // bias gradient from the same tile
-        constexpr int CC = COUT / 8;
-        const __nv_bfloat16 * gv = reinterpret_cast<const __nv_bfloat16 *>(g);
-        float acc = 0.f;
-        for (int c = 0; c < TX * TY; c++) {
-          const int x = c % TX, y = c / TX;
-          acc += __bfloat162float(gv[((y * CC + tid / 8) * TX + x) * 8 + tid % 8]);
-        }
-        bsum += acc;
-      }
-      first = false;
-      tc_fence_before();
-      __syncthreads();
-    }
-    cp_wait<0>();
-    __syncthreads();
+  if (warp < 4) {   // the accumulators start at zero
+    for (int c = 0; c < 9 * COUT; c += 16) tmem_zero<16>(tmem + ((unsigned)(warp * 32) << 16) + c);
+    tmem_wait_st();
   }
-  drain(0);
-  drain(1);
-  tc_fence_after();
-  // raw partial sums of this CTA: [a][m][co]
-  float * dst = A.part + (size_t)blockIdx.x * 9 * 128 * COUT;
-  const int m = warp * 32 + lane;
-  for (int a = 0; a < 9; a++) {
-#pragma unroll
-    for (int h = 0; h < COUT / 16; h++) {
-      float v[16];
-      tmem_ld16(tmem + ((unsigned)(warp * 32) << 16) + a * COUT + h * 16, v);
-#pragma unroll
-      for (int q = 0; q < 16; q++) dst[((size_t)a * 128 + m) * COUT + h * 16 + q] = first ? 0.f : v[q];
-    }
-  }
-  float * bdst = A.part + (size_t)gridDim.x * 9 * 128 * COUT + (size_t)blockIdx.x * COUT;
-  if (tid < COUT) bdst[tid] = bsum;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) tmem_free(tmem, L::TCOLS);
+  ConvArgs grid{};   // the cursor reads the grid only
+  grid.nx = A.nx;
+  grid.ny = A.ny;
+  grid.nz = A.nz;
+  ConvCursor cur(grid);
+  ConvSeg it;
+  // h counts steps (halo planes), g gradient tiles, over all segments: step h uses
+  // halo slot h % NS; tile g sits in slot g % NG
+  if (warp > WG_MMA) {
+    // loaders: a step's copies go out once its slots are free; the step LAG before
+    // is announced first, so that announcing never waits on MMAs
+    const int lt = tid - 32 * (WG_MMA + 1);
+    int h = 0, g = 0;
+    bool ok = true;
+    while (ok && cur.next(grid, it)) {
+      for (int p = it.z0 - 1; p <= it.z1; p++, h++) {
+        if (h >= L::LAG) {
+          cp_wait<L::LAG - 1>();
+          fence_proxy_async();
+          nn_arrive(&full[(h - L::LAG) % NS]);
+        }
+        const bool tile = p + 1 < it.z1;
+        ok = h < NS || conv_wait(&sfree[h % NS], (unsigned)((h - NS) / NS) & 1u, abort_flag);
+        if (ok && tile && g >= NG) ok = conv_wait(&gfree[g % NG], (unsigned)((g - NG) / NG) & 1u, abort_flag);
+        if (!ok) break;
+        load_wgrad_halo<CIN, COUT>(smw + (h % NS) * L::HB, A, it.x0, it.y0, wrapi(p, A.nz), lt);
+        if (tile) {
+          load_wgrad_tile<CIN, COUT>(tiles, A, it.x0, it.y0, p + 1, g % NG, lt);
+          g++;
+        }
+        cp_commit();
+      }
+    }
+    cp_wait<0>();
+    fence_proxy_async();
+    if (ok)
+      for (int q = h - L::LAG < 0 ? 0 : h - L::LAG; q < h; q++) nn_arrive(&full[q % NS]);
+    if (!ok && lane == 0) atomicOr(A.status, ST_TIMEOUT);
+  } else if (warp == WG_MMA) {
+    if (lane == 0) {
+      const unsigned sb = su32(smw), tb = su32(tiles);
+      bool ok = true;
+      int h = 0, gb = 0;   // gb: tiles of the segments before this one
+      while (ok && cur.next(grid, it)) {
+        for (int p = it.z0 - 1; p <= it.z1; p++, h++) {
+          ok = conv_wait(&full[h % NS], (unsigned)(h / NS) & 1u, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          // tiles lo .. hi of the segment that plane p meets; block z - (p - 1) of the accumulators
+          const int lo = max(p - 1, it.z0), hi = min(p + 1, it.z1 - 1), n = hi - lo + 1;
+          const unsigned bs = tb + (unsigned)(((gb + lo - it.z0) % NG) * L::GP);
+          const uint64_t bd0 = smem_desc(bs, L::GROW, TX * 16);
+          const uint64_t ad0 = smem_desc(sb + (unsigned)((h % NS) * L::HB), L::ROWB, L::CHB);
+          const unsigned d = tmem + (unsigned)((lo - (p - 1)) * COUT);
+          const uint32_t idesc = n == 1 ? instr_desc_bf16(128, COUT, 1, 1)
+                               : n == 2 ? instr_desc_bf16(128, 2 * COUT, 1, 1)
+                                        : instr_desc_bf16(128, 3 * COUT, 1, 1);
+#pragma unroll
+          for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+            for (int s = 0; s < TY / 2; s++)   // 16 cells: two y rows
+              mma_bf16(d + (unsigned)(dx * 3 * COUT), ad0 + (uint64_t)((dx * 16 + 2 * s * L::ROWB) >> 4),
+                       bd0 + (uint64_t)((2 * s * L::GROW) >> 4), idesc, true);
+          mma_commit(&sfree[h % NS]);
+          if (p - 1 >= it.z0) mma_commit(&gfree[(gb + p - 1 - it.z0) % NG]);   // tile p - 1 met its last plane
+        }
+        gb += it.z1 - it.z0;
+      }
+      if (!ok) {
+        *abort_flag = 1;
+        atomicOr(A.status, ST_TIMEOUT);
+      }
+      mma_commit(fin);   // the readout starts, and the CTA ends, after the last MMA
+    }
+    __syncwarp();
+  } else {
+    // bias gradient: every thread sums its 16-byte units (8 channels of one cell)
+    // of each tile; unit u is channel chunk (u / TX) % CG, the same for all of a thread's
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    int h = 0, g = 0;
+    bool ok = true, any = false;
+    while (ok && cur.next(grid, it)) {
+      any = true;
+      for (int p = it.z0 - 1; p <= it.z1; p++, h++) {
+        ok = conv_wait(&full[h % NS], (unsigned)(h / NS) & 1u, abort_flag);
+        if (!ok) break;
+        __syncwarp();
+        if (lane == 0) nn_arrive(&sfree[h % NS]);
+        if (p + 1 >= it.z1) continue;   // no tile comes with this step
+        static_assert(128 % (CG * TX) == 0, "one channel chunk per thread");
+#pragma unroll
+        for (int u = 0; u < TY * CG * TX / 128; u++) {
+          const int q = tid + 128 * u;
+          const uint4 w = *reinterpret_cast<const uint4 *>(tiles + (q / (CG * TX)) * L::GROW + (g % NG) * L::GP +
+                                                           (q % (CG * TX)) * 16);
+          const unsigned b[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            acc[2 * c] += __uint_as_float(b[c] << 16);
+            acc[2 * c + 1] += __uint_as_float(b[c] & 0xffff0000u);
+          }
+        }
+        __syncwarp();
+        if (lane == 0) nn_arrive(&gfree[g % NG]);
+        g++;
+      }
+    }
+    // over the warp's eight x of each chunk, then the four warps through shared memory
+    float * red = reinterpret_cast<float *>(smw + L::RED);
+    constexpr int CW = 32 / TX;   // channel chunks a warp's lanes cover at once
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+#pragma unroll
+      for (int o = 1; o < TX; o <<= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    for (int c = lane; c < COUT; c += 32) red[warp * COUT + c] = 0.f;
+    __syncwarp();
+    // chunk of lane l in warp w: ((32 w + l) / TX) % CG
+    if (lane % TX == 0) {
+      const int ch = ((tid / TX) % CG) * 8;
+#pragma unroll
+      for (int c = 0; c < 8; c++) atomicAdd(&red[warp * COUT + ch + c], acc[c]);   // CW > CG: chunks repeat
+    }
+    static_assert(CW >= 1, "lanes cover whole chunks");
+    if (!nn_mbar_wait(fin, 0)) {
+      if (lane == 0) atomicOr(A.status, ST_TIMEOUT);
+      any = false;
+    }
+    tc_fence_after();
+    // raw partial sums of this CTA: [a][m][co], a = 3 (dz + 1) + dx + 1 from the
+    // column blocks 3 (dx + 1) + 1 - dz
+    float * dst = A.part + (size_t)blockIdx.x * 9 * 128 * COUT;
+    const bool wide = (reinterpret_cast<uintptr_t>(A.part) & 15u) == 0;   // the workspace may start at any float
+    for (int a = 0; a < 9; a++) {
+      const int blk = 3 * (a % 3) + 2 - a / 3;
+#pragma unroll
+      for (int q0 = 0; q0 < COUT; q0 += 16) {
+        float v[16];
+        tmem_ld16(tmem + ((unsigned)(warp * 32) << 16) + blk * COUT + q0, v);
+        float * d = dst + ((size_t)a * 128 + tid) * COUT + q0;
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = any ? v[q] : 0.f;
+        if (wide) {
+#pragma unroll
+          for (int q = 0; q < 16; q += 4)
+            *reinterpret_cast<float4 *>(d + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 16; q++) d[q] = v[q];
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (tid < COUT) {
+    const float * red = reinterpret_cast<const float *>(smw + L::RED);
+    A.part[(size_t)gridDim.x * 9 * 128 * COUT + (size_t)blockIdx.x * COUT + tid] =
+        (red[tid] + red[COUT + tid]) + (red[2 * COUT + tid] + red[3 * COUT + tid]);
+  }
+  if (warp == WG_MMA) {
+    if (lane == 0) nn_mbar_wait(fin, 0);   // no MMA in flight when the columns are freed
+    __syncwarp();
+    tmem_free(tmem, L::TCOLS);
+  }
 }
 
 // Sum of the CTAs' raw partials into the master-layout gradients
 // dw[t][co][ci] (real channel counts) and db[co]; beta = 0 overwrites,
-// 1 accumulates.
-__global__ void wgrad_reduce_kernel(const float * __restrict__ part, int nblk, int cinp, int coutp, int cin, int cout,
-                                    float * __restrict__ dw, float * __restrict__ db, float beta) {
-  const int nw = 27 * cout * cin;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nw + cout; q += gridDim.x * blockDim.x) {
-    if (q < nw) {
-      const int ci = q % cin, co = (q / cin) % cout, t = q / (cin * cout);
-      const int dz = t / 9, dyi = (t / 3) % 3, dx = t % 3;   // dyi = dy + 1
-      const int a = dz * 3 + dx, m = (dyi * (cinp / 8) + ci / 8) * 8 + ci % 8;
-      float acc = 0.f;
-      for (int b = 0; b < nblk; b++) acc += part[(((size_t)b * 9 + a) * 128 + m) * coutp + co];
-      dw[q] = beta * dw[q] + acc;
-    } else {
-      const int co = q - nw;
-      float acc = 0.f;
-      const float * bp = part + (size_t)nblk * 9 * 128 * coutp;
-      for (int b = 0; b < nblk; b++) acc += bp[(size_t)b * coutp + co];
-      db[co] = beta * db[co] + acc;
+// 1 accumulates. A block takes 32 consecutive partial values (output channels
+// fastest, as they lie in memory), its eight warps every eighth CTA's.
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float * __restrict__ part, int nblk, int cinp,
+                                                           int coutp, int cin, int cout, float * __restrict__ dw,
+                                                           float * __restrict__ db, float beta) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int nraw = 9 * 3 * cinp * coutp;           // y shifts 0 .. 2 of the nine accumulators
+  const int q = blockIdx.x * 32 + lane;            // raw value, then the bias sums
+  const bool wt = q < nraw;
+  const int co = wt ? q % coutp : q - nraw, m = (q / coutp) % (3 * cinp), a = q / (coutp * 3 * cinp);
+  float acc = 0.f;
+  if (q < nraw + coutp) {
+    const size_t step = wt ? (size_t)9 * 128 * coutp : (size_t)coutp;
+    const float * src = wt ? part + ((size_t)a * 128 + m) * coutp + co : part + (size_t)nblk * 9 * 128 * coutp + co;
+#pragma unroll 4
+    for (int b = w; b < nblk; b += 8) acc += src[(size_t)b * step];
+  }
+  red[w][lane] = acc;
+  __syncthreads();
+  if (w != 0 || q >= nraw + coutp) return;
+  for (int r = 1; r < 8; r++) acc += red[r][lane];
+  if (wt) {
+    // accumulator row m: y shift m / cinp, input channel m % cinp; a = 3 (dz + 1) + dx + 1
+    const int ci = m % cinp, dyi = m / cinp, dz = a / 3, dx = a % 3;
+    if (ci < cin && co < cout) {
+      float * d = dw + ((size_t)(dz * 9 + dyi * 3 + dx) * cout + co) * cin + ci;
+      *d = beta * *d + acc;
     }
+  } else if (co < cout) {
+    db[co] = beta * db[co] + acc;
   }
 }
 
@@ -763,7 +875,7 @@ int launch_wgrad(WgradArgs a, int nblk, cudaStream_t st) {
   if (cudaFuncSetAttribute(conv3_wgrad_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES) !=
       cudaSuccess)
     return 1;
-  conv3_wgrad_kernel<CIN, COUT><<<nblk, NN_THREADS, L::BYTES, st>>>(a);
+  conv3_wgrad_kernel<CIN, COUT><<<nblk, WG_THREADS, L::BYTES, st>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
@@ -906,13 +1018,14 @@ int dispatch_conv3(int cin, int cout, const ConvArgs & a, cudaStream_t st) {
   return 1;
 }
 
-// weight gradient: (column tile, z chunk) work items and the CTAs over them
-void wgrad_split(int nx, int ny, int nz, int & zc, int & nitems, int & nblk) {
+// weight gradient: CTAs over the planes of all column tiles (each reads two halo
+// planes more per segment, so at least four planes apiece where nz allows)
+int wgrad_ctas(int nx, int ny, int nz) {
   const int ncol = (nx / TX) * (ny / TY);
-  zc = nz;
+  int zc = nz;
   while (zc > 4 && (long)ncol * ((nz + zc - 1) / zc) < 148L * 2) zc = (zc + 1) / 2;
-  nitems = ncol * ((nz + zc - 1) / zc);
-  nblk = nitems < 148 ? nitems : 148;
+  const int nitems = ncol * ((nz + zc - 1) / zc);
+  return nitems < 148 ? nitems : 148;
 }
 
 }  // namespace
@@ -1110,9 +1223,7 @@ int tcgpu_nn_conv3(int mode, int cin, int cout, int nx, int ny, int nz, const vo
 
 size_t tcgpu_nn_wgrad_workspace(int nx, int ny, int nz, int coutp) {
   if (nx % TX || ny % TY || nx <= 0 || ny <= 0 || nz <= 0) return 0;
-  int zc, nitems, nblk;
-  wgrad_split(nx, ny, nz, zc, nitems, nblk);
-  return (size_t)nblk * (9 * 128 + 1) * coutp * sizeof(float);
+  return (size_t)wgrad_ctas(nx, ny, nz) * (9 * 128 + 1) * coutp * sizeof(float);
 }
 
 int tcgpu_nn_conv3_wgrad(int cinp, int coutp, int cin, int cout, int nx, int ny, int nz, const void * x,
@@ -1126,8 +1237,7 @@ int tcgpu_nn_conv3_wgrad(int cinp, int coutp, int cin, int cout, int nx, int ny,
     return nn_fail("nn_conv3_wgrad: workspace smaller than tcgpu_nn_wgrad_workspace()");
   WgradArgs a{};
   a.nx = nx; a.ny = ny; a.nz = nz;
-  int nblk;
-  wgrad_split(nx, ny, nz, a.zc, a.nitems, nblk);
+  const int nblk = wgrad_ctas(nx, ny, nz);
   a.x = static_cast<const __nv_bfloat16 *>(x);
   a.dy = static_cast<const __nv_bfloat16 *>(dy);
   a.part = static_cast<float *>(workspace);
@@ -1140,8 +1250,8 @@ int tcgpu_nn_conv3_wgrad(int cinp, int coutp, int cin, int cout, int nx, int ny,
   else if (cinp == 32 && coutp == 16) rc = launch_wgrad<32, 16>(a, nblk, st);
   else if (cinp == 16 && coutp == 16) rc = launch_wgrad<16, 16>(a, nblk, st);
   if (rc) return nn_fail("nn_conv3_wgrad: unsupported channel counts or launch failure");
-  const int nred = 27 * cout * cin + cout;
-  wgrad_reduce_kernel<<<(nred + 255) / 256, 256, 0, st>>>(a.part, nblk, cinp, coutp, cin, cout, dw, db, beta);
+  const int nred = 27 * coutp * cinp + coutp;   // a multiple of 16
+  wgrad_reduce_kernel<<<(nred + 31) / 32, 256, 0, st>>>(a.part, nblk, cinp, coutp, cin, cout, dw, db, beta);
   return cudaGetLastError() == cudaSuccess ? 0 : nn_fail("nn_conv3_wgrad: reduction launch failed");
 }
 
