@@ -134,8 +134,9 @@ struct XFactors {
   double * w;               // 1 / pivot
   double * scan;            // [12][XSCAN_ROWS][32] products of f (g) over the lanes a scan level spans
   int ne;                   // elements per lane of the radial solves (warps of the predict kernel)
-  // FP32-storage contexts keep the rows of tc_march_f32.cu: f holds l_e (l_0 = 0),
-  // g the back-substitution factor u_e w_e (0 in the last row); no scan products
+  // FP32-storage contexts (tc_march_f32.cuh): f holds l_e (l_0 = 0), g the
+  // back-substitution factor u_e w_e (0 in the last row), the scan products those
+  // of -w_e l_e and -u_e w_e
   bool single;
 };
 
@@ -232,13 +233,6 @@ void launch_predict_march(const Geo & g, const Bc & bc, const Coefs & cf, const 
                           const DeltaSet & ds, const double * dtp, int rkstep, int mode, unsigned * status,
                           cudaStream_t st);
 void march_smem_limits();
-// the same for FP32-storage contexts (tc_march_f32.cu)
-void launch_predict_march32(const Geo & g, const Bc & bc, const Coefs & cf, const XFactors & xf, double nu,
-                            double kappa, const FieldBufs & in, const FieldBufs & out, const SrcBufs & ss,
-                            const DeltaSet & ds, const double * dtp, int rkstep, int mode, unsigned * status,
-                            cudaStream_t st);
-void launch_xsolve32(const Geo & g, const XFactors & xf, int rkstep, const DeltaSet & ds, cudaStream_t st);
-void march32_smem_limits();
 // radial implicit solves of the delta buffers, lines of up to 1024 points
 // (after the predict's tile mode, nx > 256)
 void launch_xsolve(const Geo & g, const XFactors & xf, int rkstep, const DeltaSet & ds, cudaStream_t st);

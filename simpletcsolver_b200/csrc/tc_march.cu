@@ -10,7 +10,7 @@ namespace tcgpu {
 // tile mode above leaves its increments unsolved): one warp per (variable,
 // j, k) line of the delta buffers, staged in shared memory, with the factor
 // rows and scans of the march kernel (solve_line).
-template <int E>
+template <int E, bool SINGLE>
 __global__ void __launch_bounds__(256) xsolve_kernel(Geo g, XFactors xf, int rk, DeltaSet ds) {
   extern __shared__ double xs_stage[];
   constexpr int SL = 32 * E + 32;
@@ -25,9 +25,9 @@ __global__ void __launch_bounds__(256) xsolve_kernel(Geo g, XFactors xf, int rk,
   double * d = ds.d[v] + (size_t)jk * n;   // packed layout: line (j, k) holds n values
   for (int e = lane; e < 32 * E; e += 32) sb[march::spad<E>(e)] = e < n ? d[e] : 0.;
   __syncwarp();
-  march::LineFactors<E> factors;
+  march::LineFactors<E, SINGLE> factors;
   factors.load(xf, rk, v, lane);
-  march::solve_lines<E, 1>(sb, 0, factors, lane);
+  march::solve_lines<E, 1, SINGLE>(sb, 0, factors, lane);
   __syncwarp();
   for (int e = lane; e < n; e += 32) d[e] = sb[march::spad<E>(e)];
 }
@@ -73,13 +73,19 @@ void launch_predict_march(const Geo & g, const Bc & bc, const Coefs & cf, const 
                           double kappa, const FieldBufs & in, const FieldBufs & out, const SrcBufs & ss,
                           const DeltaSet & ds, const double * dtp, int rkstep, int mode, unsigned * status,
                           cudaStream_t st) {
+  const int mask = (bc.implicit[0] ? 1 : 0) | (bc.implicit[1] ? 2 : 0) | (bc.implicit[2] ? 4 : 0);
+  const bool tiles = g.nx > 256;   // wider than a CTA's field threads: increments only, solved afterwards
   if (in.bytes == 4) {
-    launch_predict_march32(g, bc, cf, xf, nu, kappa, in, out, ss, ds, dtp, rkstep, mode, status, st);
+    march::Args<float> A{g, bc, cf, xf, nu, kappa, in.as<float>(), out.as<float>(), ss.as<float>(), ds, rkstep, mode, 0,
+                         status};
+    if (tiles) A.mode = PREDICT_DELTA;
+    if (mask == 1 && !tiles) march::launch<1, float>(A, tiles, dtp, st);
+    else if (mask == 7 && !tiles) march::launch<7, float>(A, tiles, dtp, st);
+    else if (mask == 0 && !tiles) march::launch<0, float>(A, tiles, dtp, st);
+    else march::launch<-1, float>(A, tiles, dtp, st);
     return;
   }
   using T = double;
-  const int mask = (bc.implicit[0] ? 1 : 0) | (bc.implicit[1] ? 2 : 0) | (bc.implicit[2] ? 4 : 0);
-  const bool tiles = g.nx > 256;   // wider than a CTA's field threads: increments only, solved afterwards
   march::Args<T> A{g, bc, cf, xf, nu, kappa, in.as<T>(), out.as<T>(), ss.as<T>(), ds, rkstep, mode, 0, status};
   if (tiles) A.mode = PREDICT_DELTA;
   // the common masks have instances of their own; the others, and tiles, read the
@@ -114,19 +120,18 @@ __global__ void wait_selftest_kernel(unsigned * status) {
 void launch_wait_selftest(unsigned * status, cudaStream_t st) { wait_selftest_kernel<<<1, 64, 0, st>>>(status); }
 
 void launch_xsolve(const Geo & g, const XFactors & xf, int rkstep, const DeltaSet & ds, cudaStream_t st) {
-  if (xf.single) {
-    launch_xsolve32(g, xf, rkstep, ds, st);
-    return;
-  }
   const long long lines = 4LL * g.ny * g.nz;
   const unsigned blocks = (unsigned)((lines + 7) / 8);
-  if (xf.ne <= 16) xsolve_kernel<16><<<blocks, 256, 8 * (32 * 16 + 32) * sizeof(double), st>>>(g, xf, rkstep, ds);
-  else xsolve_kernel<32><<<blocks, 256, 8 * (32 * 32 + 32) * sizeof(double), st>>>(g, xf, rkstep, ds);
+  const size_t smem = 8 * (32 * xf.ne + 32) * sizeof(double);
+  if (xf.ne == 16)
+    (xf.single ? xsolve_kernel<16, true> : xsolve_kernel<16, false>)<<<blocks, 256, smem, st>>>(g, xf, rkstep, ds);
+  else
+    (xf.single ? xsolve_kernel<32, true> : xsolve_kernel<32, false>)<<<blocks, 256, smem, st>>>(g, xf, rkstep, ds);
 }
 
 void march_smem_limits() {
-  cudaFuncSetAttribute(xsolve_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (32 * 32 + 32) * 8);
-  march32_smem_limits();
+  for (auto k : {xsolve_kernel<32, true>, xsolve_kernel<32, false>})
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (32 * 32 + 32) * 8);
 }
 
 }  // namespace tcgpu

@@ -146,9 +146,8 @@ struct Bars {
 // ------------------------------------------------------------ coefficients
 // Products of the metric tables taken once on the host (the P_* tables), each
 // spelled out below where it is used; loaded once per thread (they depend on i
-// only) with the diffusivities folded in. C is the arithmetic type of the
-// right-hand sides: double, or float in the FP32-storage mode (the increments,
-// the radial solves and the update stay double).
+// only) with the diffusivities folded in. (FP32-storage contexts have sides of
+// their own: tc_march_f32.cuh.)
 template <class C>
 struct CoefA {
   C xa1, xa2, xa3, yb1, yb2, zc1, zc2, h1, h2;        // ux advection, centrifugal term
@@ -461,7 +460,9 @@ __device__ __forceinline__ int spad(int e) { return e + e / E; }
 // lines at a time (stride doubles apart) hide the chains' and the shuffles' latency.
 // Elements from n on have f = g = w = 0. Per plane of two 256-point lines: 1.9k
 // cycles, against 4.2k with the factor rows read and multiplied out for each line.
-template <int E>
+// SINGLE (FP32-storage contexts) keeps the former order of roundings: r_m w_m
+// first, f_m = -w_m l_m and g_m = -v_m with the rows' l, w, v (XFactors::single).
+template <int E, bool SINGLE>
 struct LineFactors {
   double f[E], g[E], w[E], up[5], down[5];
   // rows are interleaved: element lane E + m at m 32 + lane
@@ -473,6 +474,10 @@ struct LineFactors {
       f[m] = LD(xf.f + o + m * 32);
       g[m] = LD(xf.g + o + m * 32);
       w[m] = LD(xf.w + o + m * 32);
+      if (SINGLE) {
+        f[m] = __dmul_rn(-w[m], f[m]);
+        g[m] = -g[m];
+      }
     }
 #pragma unroll
     for (int q = 0; q < 5; q++) {
@@ -481,44 +486,44 @@ struct LineFactors {
     }
   }
 };
-template <int E, int LN>
-__device__ __forceinline__ void solve_lines(double * sb, int stride, const LineFactors<E> & x, int lane) {
+template <int E, int LN, bool SINGLE>
+__device__ __forceinline__ void solve_lines(double * sb, int stride, const LineFactors<E, SINGLE> & x, int lane) {
   double r[LN][E], B[LN];
   sb += spad<E>(lane * E);   // the lane's E elements are consecutive
 #pragma unroll
   for (int n = 0; n < LN; n++)
 #pragma unroll
-    for (int m = 0; m < E; m++) r[n][m] = sb[n * stride + m];
+    for (int m = 0; m < E; m++) r[n][m] = SINGLE ? __dmul_rn(x.w[m], sb[n * stride + m]) : sb[n * stride + m];
 #pragma unroll
   for (int n = 0; n < LN; n++) {
     B[n] = r[n][0];
 #pragma unroll
-    for (int m = 1; m < E; m++) B[n] = x.f[m] * B[n] + r[n][m];
+    for (int m = 1; m < E; m++) B[n] = fma(x.f[m], B[n], r[n][m]);
   }
 #pragma unroll
   for (int q = 0; q < 5; q++)
 #pragma unroll
-    for (int n = 0; n < LN; n++) B[n] += x.up[q] * __shfl_up_sync(0xffffffffu, B[n], 1 << q);
+    for (int n = 0; n < LN; n++) B[n] = fma(x.up[q], __shfl_up_sync(0xffffffffu, B[n], 1 << q), B[n]);
 #pragma unroll
   for (int n = 0; n < LN; n++) {
     double p = __shfl_up_sync(0xffffffffu, B[n], 1);   // lane 0: f[0] = 0
 #pragma unroll
-    for (int m = 0; m < E; m++) p = r[n][m] += x.f[m] * p;
+    for (int m = 0; m < E; m++) p = r[n][m] = fma(x.f[m], p, r[n][m]);
     B[n] = r[n][E - 1];
 #pragma unroll
-    for (int m = E - 2; m >= 0; m--) B[n] = x.g[m] * B[n] + r[n][m];
+    for (int m = E - 2; m >= 0; m--) B[n] = fma(x.g[m], B[n], r[n][m]);
   }
 #pragma unroll
   for (int q = 0; q < 5; q++)
 #pragma unroll
-    for (int n = 0; n < LN; n++) B[n] += x.down[q] * __shfl_down_sync(0xffffffffu, B[n], 1 << q);
+    for (int n = 0; n < LN; n++) B[n] = fma(x.down[q], __shfl_down_sync(0xffffffffu, B[n], 1 << q), B[n]);
 #pragma unroll
   for (int n = 0; n < LN; n++) {
     double p = __shfl_down_sync(0xffffffffu, B[n], 1);   // lane 31: g of the last element is 0
 #pragma unroll
     for (int m = E - 1; m >= 0; m--) {
-      p = r[n][m] + x.g[m] * p;
-      sb[n * stride + m] = x.w[m] * p;
+      p = fma(x.g[m], p, r[n][m]);
+      sb[n * stride + m] = SINGLE ? p : x.w[m] * p;
     }
   }
 }
@@ -633,7 +638,7 @@ template <class L, int GRP, int IMPL, class T, bool TILE>
 struct Group {
   static constexpr bool D64 = L::D64;
   static constexpr int VA = GRP == 0 ? VUX : VUY, VB = GRP == 0 ? VT : VUZ;
-  using C = T;   // the right-hand sides' arithmetic follows the storage
+  using C = T;
   typename std::conditional<GRP == 0, CoefA<C>, CoefB<C>>::type q;
   Share<C> ua, ub;           // the lower z faces' shares of the next plane to form
   T * na, * nb;              // new source terms of the pair's first line, next plane
@@ -816,7 +821,7 @@ __device__ __forceinline__ void solves(const Args<T> & A, const Box & x, char * 
   copies.old_terms(x, olds, v, bars, abort_flag);
   const Dirs<IMPL> im(A.bc);
   const bool solve_x = !TILE && im.x;
-  LineFactors<E> factors;
+  LineFactors<E, sizeof(T) == 4> factors;
   if (solve_x) factors.load(A.xf, A.rkstep, v, lane);
   const int i0 = v == VUX ? 2 : 1;              // radial index of unknown 0
   const int n = v == VUX ? nx - 1 : nx;         // unknowns of a line
@@ -843,7 +848,7 @@ __device__ __forceinline__ void solves(const Args<T> & A, const Box & x, char * 
     const T * us = reinterpret_cast<const T *>(ring + (size_t)slot_of<L>(k, x.k0) * L::SLOT) + u0;
     // all lines of the variable at once (those past ny in the last CTA are zero)
     if (solve_x) {
-      solve_lines<E, L::JT>(sd, 4 * L::SL, factors, lane);
+      solve_lines<E, L::JT, sizeof(T) == 4>(sd, 4 * L::SL, factors, lane);
       __syncwarp();
     }
 #pragma unroll 1

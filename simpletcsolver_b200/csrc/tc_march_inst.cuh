@@ -2,6 +2,7 @@
 #pragma once
 #include <atomic>
 
+#include "tc_march_f32.cuh"
 #include "tc_march_launch.cuh"
 
 namespace tcgpu {
@@ -31,10 +32,15 @@ void launch_one(Args<T> A, const double * dtp, cudaStream_t st) {
 
 template <int IMPL, class T>
 void launch(Args<T> A, bool tiles, const double * dtp, cudaStream_t st) {
-  if constexpr (IMPL < 0 || IMPL == 1)
+  if constexpr (IMPL < 0 || (IMPL == 1 && sizeof(T) == 8))
     if (tiles) return launch_one<8, 1, 1, IMPL, T, true>(A, dtp, st);
-  switch (predict_warps(A.g.nx)) {
-#define X(NW, PAIRS, NG) case NW: return launch_one<NW, PAIRS, NG, IMPL, T, false>(A, dtp, st);
+  switch (sizeof(T) == 8 ? predict_warps(A.g.nx) : predict_warps32(A.g.nx)) {
+#define X(NW, PAIRS, NG)                                                   \
+  case NW:                                                                 \
+    if constexpr (sizeof(T) == 8 || (NW & (NW - 1)) == 0) /* predict_warps32 */ \
+      return launch_one<NW, PAIRS, NG, IMPL, T, false>(A, dtp, st);          \
+    else                                                                     \
+      return;
     TC_MARCH_INSTANCES(X)
 #undef X
   }

@@ -1,0 +1,8 @@
+#include "tc_march_inst.cuh"
+
+namespace tcgpu {
+namespace march {
+template void launch<1, float>(Args<float>, bool, const double *, cudaStream_t);
+template void launch<7, float>(Args<float>, bool, const double *, cudaStream_t);
+}  // namespace march
+}  // namespace tcgpu

@@ -1116,7 +1116,7 @@ static int mixed_lines(int n, int cap) {
 
 // --------------------------------------------------------------- direct DFTs
 // FP32-storage contexts take direct transforms for lengths that are not powers of
-// two (their results hold to the last stored bit; tc_march_f32.cu): each
+// two (their results hold to the last stored bit; tc_march_f32.cuh): each
 // output wavenumber is the sum over the line with twiddles tw[(j m) mod N] =
 // exp(-2 pi i (j m mod N) / N) from the same tables. O(N^2) per line, FP64
 // accumulation, FFTW's conventions (unnormalised, r2c keeps N/2+1 terms, c2r

@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) xfactor_kernel(XFactors xf, const double 
 }
 
 // The rows of FP32-storage contexts: l_e, w_e and v_e = u_e w_e from the division
-// recurrence of gtsv, in its order of roundings (tc_march_f32.cu). The rows are
+// recurrence of gtsv, in its order of roundings (tc_march_f32.cuh). The rows are
 // staged in shared memory by the block, so that only the recurrence is serial.
 __global__ void __launch_bounds__(256) xfactor32_kernel(XFactors xf, const double * __restrict__ dtp, double nu, double kappa) {
   __shared__ double sl[XF_MAX], sc[XF_MAX], su[XF_MAX];   // l; c, then w; u, then v
@@ -118,6 +118,22 @@ __global__ void __launch_bounds__(256) xfactor32_kernel(XFactors xf, const doubl
     xf.f[row + pe] = e > 0 ? sl[e] : 0.;
     xf.w[row + pe] = sc[e];
     xf.g[row + pe] = su[e];
+  }
+  if (tid < 32) {   // products of -w l and of -v over the lanes a scan level spans
+    double pfw = 1., pbw = 1.;
+    for (int m = 0; m < ne; m++) {
+      const int e = tid * ne + m;
+      pfw = __dmul_rn(e < n ? __dmul_rn(-sc[e], e > 0 ? sl[e] : 0.) : -0., pfw);
+    }
+    for (int m = ne - 1; m >= 0; m--) pbw = __dmul_rn(tid * ne + m < n ? -su[tid * ne + m] : -0., pbw);
+    double * s = xf.scan + (size_t)rv * XSCAN_ROWS * 32;
+    for (int q = 0; q < 5; q++) {
+      s[q * 32 + tid] = tid >= (1 << q) ? pfw : 0.;
+      s[(5 + q) * 32 + tid] = tid + (1 << q) < 32 ? pbw : 0.;
+      const double a = __shfl_up_sync(0xffffffffu, pfw, 1 << q), b = __shfl_down_sync(0xffffffffu, pbw, 1 << q);
+      if (tid >= (1 << q)) pfw = __dmul_rn(pfw, a);
+      if (tid + (1 << q) < 32) pbw = __dmul_rn(pbw, b);
+    }
   }
 }
 
@@ -497,6 +513,7 @@ void launch_yzfactors(const Geo & g, const YZFactors & yf, const double * dtp, d
 }
 
 // ------------------------------------------------------------ launchers
+// FP32-storage contexts: powers of two (their solves hold to the last bit)
 int predict_warps32(int nx) {
   int w = 1;
   while (32 * w < nx) w *= 2;
