@@ -458,6 +458,10 @@ static int build_tables(Ctx & c, const domain_t * d) {
     yf.vz = dalloc(c, 12 * (size_t)nz);
     yf.wz = dalloc(c, 12 * (size_t)nz);
     yf.q1z = dalloc(c, 12 * (size_t)nz);
+    // FP64 contexts: solves with shared factors where the lines have them
+    if (c.sb == 8 && c.bc.implicit[1] && yf.uniform_y && shared_lines_table(ny)) yf.ty = dalloc(c, shared_lines_table(ny));
+    if (c.sb == 8 && c.bc.implicit[2] && shared_lines_table(nz)) yf.tz = dalloc(c, shared_lines_table(nz));
+    cudaGetLastError();   // without a table the general solves run
   }
 
   // Poisson tables (compute_potential.c:173-211, 311-349)
@@ -579,7 +583,7 @@ static void allow_smem() {
   std::lock_guard<std::mutex> lk(m);
   if (std::find(done.begin(), done.end(), dev) != done.end()) return;
   poisson_smem_limits();
-  march_smem_limits();
+  allow_lines_smem();
   allow_periodic_lines_smem();
   done.push_back(dev);
 }
@@ -717,7 +721,9 @@ static void * s_old(Ctx & c, int v, int rk) { return c.src[v][rk == 1 ? 0 : 1]; 
 
 static void enqueue_factors(Ctx & c) {
   if (c.bc.implicit[0]) { launch_xfactors(c.xf, c.dtp, c.nu, c.kappa, c.st); mark(TCGPU_K_FACTORS); }
-  if (c.bc.implicit[1] || c.bc.implicit[2]) { launch_yzfactors(c.g, c.yf, c.dtp, c.nu, c.kappa, c.st); mark(TCGPU_K_FACTORS); }
+  const YZFactors & yf = c.yf;
+  if (yf.ty || yf.tz) { launch_shared_factors(c.g, yf, c.dtp, c.nu, c.kappa, c.st); mark(TCGPU_K_FACTORS); }
+  if ((c.bc.implicit[1] && !yf.ty) || (c.bc.implicit[2] && !yf.tz)) { launch_yzfactors(c.g, yf, c.dtp, c.nu, c.kappa, c.st); mark(TCGPU_K_FACTORS); }
 }
 
 static void enqueue_predict(Ctx & c, int rk) {
@@ -741,11 +747,25 @@ static void enqueue_predict(Ctx & c, int rk) {
   } else {
     predict(PREDICT_DELTA);
     mark(TCGPU_K_PREDICT);
-    if (tiles && c.bc.implicit[0]) { launch_xsolve(c.g, c.xf, rk, c.ds, c.st); mark(TCGPU_K_YZSOLVE); }
-    if (iy) { launch_ysolve(c.g, c.yf, rk, c.ds, c.st); mark(TCGPU_K_YZSOLVE, 4); }
-    if (iz) { launch_zsolve(c.g, c.yf, rk, c.ds, c.st); mark(TCGPU_K_YZSOLVE, 4); }
-    launch_apply(c.g, c.bc, in, out, c.ds, c.st);
-    mark(TCGPU_K_APPLY);
+    // the last implicit direction's solve stores the updated fields itself where
+    // it can; otherwise the update follows
+    bool updated = false;
+    if (tiles && c.bc.implicit[0]) {
+      updated = !iy && !iz;
+      launch_xsolve(c.g, c.bc, c.xf, rk, c.ds, in, out, updated, c.st);
+      mark(TCGPU_K_YZSOLVE);
+    }
+    if (iy && c.yf.ty) {
+      updated = !iz;
+      launch_shared_lines(c.g, c.bc, c.ds, in, out, c.yf.ty, rk, false, updated, c.st);
+      mark(TCGPU_K_YZSOLVE);
+    } else if (iy) { launch_ysolve(c.g, c.yf, rk, c.ds, c.st); mark(TCGPU_K_YZSOLVE, 4); }
+    if (iz && c.yf.tz) {
+      updated = true;
+      launch_shared_lines(c.g, c.bc, c.ds, in, out, c.yf.tz, rk, true, updated, c.st);
+      mark(TCGPU_K_YZSOLVE);
+    } else if (iz) { launch_zsolve(c.g, c.yf, rk, c.ds, c.st); mark(TCGPU_K_YZSOLVE, 4); }
+    if (!updated) { launch_apply(c.g, c.bc, in, out, c.ds, c.st); mark(TCGPU_K_APPLY); }
   }
   c.cur ^= 1;
 }

@@ -163,6 +163,8 @@ struct YZFactors {
   double * vz;              // [12][nz]
   double * wz;
   double * q1z;
+  double * ty;              // tables of the shared-factor solves, null where they do not apply
+  double * tz;
 };
 
 // Poisson solver state.
@@ -232,10 +234,10 @@ void launch_predict_march(const Geo & g, const Bc & bc, const Coefs & cf, const 
                           double kappa, const FieldBufs & in, const FieldBufs & out, const SrcBufs & ss,
                           const DeltaSet & ds, const double * dtp, int rkstep, int mode, unsigned * status,
                           cudaStream_t st);
-void march_smem_limits();
 // radial implicit solves of the delta buffers, lines of up to 1024 points
 // (after the predict's tile mode, nx > 256)
-void launch_xsolve(const Geo & g, const XFactors & xf, int rkstep, const DeltaSet & ds, cudaStream_t st);
+void launch_xsolve(const Geo & g, const Bc & bc, const XFactors & xf, int rkstep, const DeltaSet & ds,
+                   const FieldBufs & in, const FieldBufs & out, bool update, cudaStream_t st);
 // one CTA whose mbarrier wait can never complete: sets ST_TIMEOUT in *status
 void launch_wait_selftest(unsigned * status, cudaStream_t st);
 void launch_xfactors(const XFactors & xf, const double * dtp, double nu, double kappa, cudaStream_t st);
@@ -245,6 +247,16 @@ void launch_yzfactors(const Geo & g, const YZFactors & yf, const double * dtp, d
 void launch_ysolve(const Geo & g, const YZFactors & yf, int rkstep, const DeltaSet & ds, cudaStream_t st);
 void launch_zsolve(const Geo & g, const YZFactors & yf, int rkstep, const DeltaSet & ds, cudaStream_t st);
 void allow_periodic_lines_smem();
+void allow_lines_smem();
+// Periodic solves whose lines share their factors (FP64 contexts; z, and y where
+// YZFactors::uniform_y): doubles of a direction's table (0: lines of n points are
+// not handled), the tables YZFactors::ty and tz (null: not wanted), and the solves of one
+// direction, with the update into out in the last one
+size_t shared_lines_table(int n);
+void launch_shared_factors(const Geo & g, const YZFactors & yf, const double * dtp, double nu, double kappa,
+                           cudaStream_t st);
+void launch_shared_lines(const Geo & g, const Bc & bc, const DeltaSet & ds, const FieldBufs & in, const FieldBufs & out,
+                         const double * table, int rkstep, bool z, bool update, cudaStream_t st);
 
 // optional per-launch callback of the host's kernel accounting
 struct PoissonMarks {

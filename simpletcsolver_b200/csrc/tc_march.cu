@@ -1,36 +1,9 @@
 // Launchers of the predict stage (tc_march.cuh): the choice of the instance and
-// of the planes per CTA, the radial solves of lines longer than a CTA, and the
-// self-test of the kernels' bounded waits.
+// of the planes per CTA, and the self-test of the kernels' bounded waits.
 #include "tc_march.cuh"
 #include "tc_march_launch.cuh"
 
 namespace tcgpu {
-
-// Radial implicit solves of lines longer than one CTA's field threads (the
-// tile mode above leaves its increments unsolved): one warp per (variable,
-// j, k) line of the delta buffers, staged in shared memory, with the factor
-// rows and scans of the march kernel (solve_line).
-template <int E, bool SINGLE>
-__global__ void __launch_bounds__(256) xsolve_kernel(Geo g, XFactors xf, int rk, DeltaSet ds) {
-  extern __shared__ double xs_stage[];
-  constexpr int SL = 32 * E + 32;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const long long lines = (long long)g.ny * g.nz;
-  const long long q = (long long)blockIdx.x * 8 + w;   // (variable, line)
-  if (q >= 4 * lines) return;                          // whole warps
-  const int v = (int)(q / lines);
-  const long long jk = q % lines;
-  const int n = xf.n[v];
-  double * sb = xs_stage + (size_t)w * SL;
-  double * d = ds.d[v] + (size_t)jk * n;   // packed layout: line (j, k) holds n values
-  for (int e = lane; e < 32 * E; e += 32) sb[march::spad<E>(e)] = e < n ? d[e] : 0.;
-  __syncwarp();
-  march::LineFactors<E, SINGLE> factors;
-  factors.load(xf, rk, v, lane);
-  march::solve_lines<E, 1, SINGLE>(sb, 0, factors, lane);
-  __syncwarp();
-  for (int e = lane; e < n; e += 32) d[e] = sb[march::spad<E>(e)];
-}
 
 // Planes per CTA of a marching launch of `columns` CTAs per plane chunk: the
 // divisor of nz (up to TC_MARCH_KC) with the least waves x (planes +
@@ -118,20 +91,5 @@ __global__ void wait_selftest_kernel(unsigned * status) {
 }
 
 void launch_wait_selftest(unsigned * status, cudaStream_t st) { wait_selftest_kernel<<<1, 64, 0, st>>>(status); }
-
-void launch_xsolve(const Geo & g, const XFactors & xf, int rkstep, const DeltaSet & ds, cudaStream_t st) {
-  const long long lines = 4LL * g.ny * g.nz;
-  const unsigned blocks = (unsigned)((lines + 7) / 8);
-  const size_t smem = 8 * (32 * xf.ne + 32) * sizeof(double);
-  if (xf.ne == 16)
-    (xf.single ? xsolve_kernel<16, true> : xsolve_kernel<16, false>)<<<blocks, 256, smem, st>>>(g, xf, rkstep, ds);
-  else
-    (xf.single ? xsolve_kernel<32, true> : xsolve_kernel<32, false>)<<<blocks, 256, smem, st>>>(g, xf, rkstep, ds);
-}
-
-void march_smem_limits() {
-  for (auto k : {xsolve_kernel<32, true>, xsolve_kernel<32, false>})
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * (32 * 32 + 32) * 8);
-}
 
 }  // namespace tcgpu

@@ -2,9 +2,11 @@
 //
 // xfactor_kernel    line-independent Thomas factors of the radial implicit
 //                   systems (I - k L_x) for the three substeps, from dt on the device.
-// apply_kernel      u + delta after the y / z solves (planar configuration).
-// ysolve/zsolve     periodic (Sherman-Morrison, src/tdm.c:66-106) solves in y
-//                   and z for the planar configuration, one thread per line.
+// apply_kernel      u + delta where no line solve stores it (tc_lines.cu).
+// periodic_lines, ysolve, zsolve
+//                   periodic (Sherman-Morrison, src/tdm.c:66-106) solves in y and z
+//                   that tc_lines.cu does not take: factors that depend on the
+//                   radial index, FP32 storage, lines of more than 1024 points.
 #include "tc_common.cuh"
 #include "tc_kernels.h"
 
@@ -252,7 +254,8 @@ __global__ void zsolve_kernel(Geo g, YZFactors yf, int rkstep, int var,
 }
 
 // ------------------------------------------------------------ periodic solves, one warp per line
-// The same solves for lines of N = 32 E points: a CTA takes a tile of PT
+// The same solves for lines of N = 32 E points, factors per radial index or one set
+// (FP32 storage): a CTA takes a tile of PT
 // consecutive radial indices of one plane (y lines) or one row (z lines) into
 // shared memory with coalesced loads, and each warp solves whole lines with
 // the forward and backward Thomas recurrences written as affine maps
@@ -520,10 +523,10 @@ int predict_warps32(int nx) {
   return w;
 }
 
-// warps of the predict kernel per radial line: the instances of tc_march_inst.cuh,
-// powers of two for lines longer than 256 points (the line kernel's elements per lane)
+// warps of the predict kernel per radial line: the instances of tc_march_inst.cuh;
+// beyond 256 points the elements per lane of xsolve_kernel
 int predict_warps(int nx) {
-  for (int w : {1, 2, 3, 4, 6, 8, 16})
+  for (int w : {1, 2, 3, 4, 6, 8, 12, 16, 24})
     if (32 * w >= nx) return w;
   return 32;
 }
