@@ -5,7 +5,8 @@
 //                    :382-425) fused with the real-to-complex DFT along y; two real
 //                    lines travel as one complex FFT and are separated afterwards
 //   fftz_kernel      complex DFT along z, forward (-1) or backward (+1), in place
-//   tdm_kernel       per wavenumber pair (ky, kz) the radial Thomas solve with
+//   tdm_lines_kernel, tdm_kernel
+//                    per wavenumber pair (ky, kz) the radial Thomas solve with
 //                    c_i = -l_i - u_i + ey/hyxc_i^2 + ez/hz^2 and Neumann ends
 //                    (:445-488); the singular (0, 0) system is solved with its last
 //                    unknown pinned to zero
@@ -19,9 +20,12 @@
 // registers (N = 1024: passes of 16, 16, 4), twiddles exp(-2 pi i m / N)
 // tabulated on the host from libm.
 //
+// Other lengths: the mixed-radix kernels of tc_fft_mixed.cuh (FP64 contexts), direct
+// sums (FP32 storage).
+//
 // Spectral layout: spec[i][kz][ky] (ky fastest), so the y and z transforms read
-// and write rows of contiguous wavenumbers and the radial solve, one thread per
-// (kz, ky) line, walks i with fully coalesced steps.
+// and write rows of contiguous wavenumbers and the radial solve, a tile of
+// consecutive ky per CTA or one thread per (kz, ky) line, walks i with coalesced steps.
 #include <type_traits>
 
 #include "tc_common.cuh"
@@ -1121,98 +1125,167 @@ static int mixed_lines(int n, int cap) {
 // exp(-2 pi i (j m mod N) / N) from the same tables. O(N^2) per line, FP64
 // accumulation, FFTW's conventions (unnormalised, r2c keeps N/2+1 terms, c2r
 // ignores the imaginary parts of the DC and Nyquist terms).
+// A CTA takes L lines: a thread sums one wavenumber of all of them, so that a twiddle
+// (a gather from shared memory) serves L lines, whose values it reads as broadcasts.
+// Bound: the FP64 pipe, 2 multiply-adds a term in y and 4 in z. With one line per CTA
+// and the twiddles gathered from global memory a step of 96 x 180 x 120 took 3.16 ms,
+// 1.48 here.
 
-// divergence (as div_ffty_kernel) of one (i, k) line into shared memory, then
-// its r2c transform along y
-template <class T, class Z>
-__global__ void div_dfty_kernel(Geo g, Coefs cf, Poisson ps, const T * __restrict__ ux, const T * __restrict__ uy,
-                                const T * __restrict__ uz, const double * __restrict__ dtp, int rkstep) {
-  extern __shared__ double line[];
+// lines per CTA: as many as fit the default shared memory beside the twiddles and
+// leave a CTA for every SM
+static int dft_lines(int n, int bytes, long long lines) {
+  int L = 8;
+  while (L > 1 && ((size_t)n * (sizeof(double2) + (size_t)L * bytes) > 48 * 1024 || lines / L < 148)) L >>= 1;
+  return L;
+}
+
+// divergence (as div_ffty_kernel) of the lines (i0 .. i0 + L - 1, k) into shared
+// memory, then their r2c transforms along y
+template <int L, class T, class Z>
+__global__ void __launch_bounds__(128) div_dfty_kernel(Geo g, Coefs cf, Poisson ps, const T * __restrict__ ux,
+                                                       const T * __restrict__ uy, const T * __restrict__ uz,
+                                                       const double * __restrict__ dtp, int rkstep) {
+  extern __shared__ double2 tw[];
   const int ny = g.ny, nz = g.nz, nyh = ps.nyh;
-  const int i = blockIdx.x + 1, k = blockIdx.y + 1;
+  const int i0 = blockIdx.x * L + 1, k = blockIdx.y + 1;
+  double * const line = reinterpret_cast<double *>(tw + ny);   // [j][line]
   const double prefactor = 1. / (rk_gamma(rkstep) * (*dtp)) / (1. * ny * nz);
-  const double jxm = __ldg(cf.c_jf + i), jxp = __ldg(cf.c_jf + i + 1);
-  const double jy = __ldg(cf.c_e1 + i), jz = __ldg(cf.c_e2 + i), ijd = __ldg(cf.c_invjdxc + i);
-  for (int j = threadIdx.x + 1; j <= ny; j += blockDim.x) {
+  for (int j = threadIdx.x; j < ny; j += blockDim.x) tw[j] = ps.tw_y[j];
+  for (int q = threadIdx.x; q < ny * L; q += blockDim.x) {
+    const int i = i0 + q % L, j = q / L + 1;
+    if (i > g.nx) { line[q] = 0.; continue; }
+    const double jxm = __ldg(cf.c_jf + i), jxp = __ldg(cf.c_jf + i + 1);
+    const double jy = __ldg(cf.c_e1 + i), jz = __ldg(cf.c_e2 + i), ijd = __ldg(cf.c_invjdxc + i);
     const double div = ijd * (
         -jxm * (double)ux[sidx_f<T>(g, i, j, k)] + jxp * (double)ux[sidx_f<T>(g, i + 1, j, k)]
         - jy * (double)uy[sidx_c<T>(g, i, j, k)] + jy * (double)uy[sidx_c<T>(g, i, j + 1, k)]
         - jz * (double)uz[sidx_c<T>(g, i, j, k)] + jz * (double)uz[sidx_c<T>(g, i, j, k + 1)]);
-    line[j - 1] = prefactor * div;
+    line[q] = prefactor * div;
   }
   __syncthreads();
-  Z * out = static_cast<Z *>(ps.spec) + ((size_t)(i - 1) * nz + (k - 1)) * nyh;
+  Z * const out = static_cast<Z *>(ps.spec) + ((size_t)(i0 - 1) * nz + (k - 1)) * nyh;
   for (int m = threadIdx.x; m < nyh; m += blockDim.x) {
-    double re = 0., im = 0.;
+    double re[L] = {}, im[L] = {};
     int q = 0;   // j m mod ny
     for (int j = 0; j < ny; j++) {
-      const double2 w = ps.tw_y[q];
-      re += line[j] * w.x;
-      im += line[j] * w.y;
+      const double2 w = tw[q];
+#pragma unroll
+      for (int l = 0; l < L; l++) {
+        re[l] += line[j * L + l] * w.x;
+        im[l] += line[j * L + l] * w.y;
+      }
       q += m;
       if (q >= ny) q -= ny;
     }
-    zput(out + m, make_double2(re, im));
+#pragma unroll
+    for (int l = 0; l < L; l++)
+      if (i0 + l <= g.nx) zput(out + (size_t)l * nz * nyh + m, make_double2(re[l], im[l]));
   }
 }
 
-// complex transform along z of the columns (i, ky), in place; SIGN -1 forward
-template <int SIGN, class Z>
-__global__ void dftz_kernel(Geo g, Poisson ps) {
-  extern __shared__ double2 col[];
+// complex transform along z of the columns (i, ky0 .. ky0 + L - 1), in place;
+// SIGN -1 forward
+template <int L, int SIGN, class Z>
+__global__ void __launch_bounds__(128) dftz_kernel(Geo g, Poisson ps) {
+  extern __shared__ double2 tw[];
   const int nz = g.nz, nyh = ps.nyh;
-  const int ky = blockIdx.x, i = blockIdx.y + 1;
-  Z * base = static_cast<Z *>(ps.spec) + (size_t)(i - 1) * nz * nyh + ky;
-  for (int k = threadIdx.x; k < nz; k += blockDim.x) col[k] = zget(base + (size_t)k * nyh);
+  const int ky0 = blockIdx.x * L, i = blockIdx.y + 1;
+  double2 * const col = tw + nz;   // [k][column]
+  Z * const base = static_cast<Z *>(ps.spec) + (size_t)(i - 1) * nz * nyh + ky0;
+  for (int k = threadIdx.x; k < nz; k += blockDim.x) tw[k] = ps.tw_z[k];
+  for (int q = threadIdx.x; q < nz * L; q += blockDim.x)
+    col[q] = ky0 + q % L < nyh ? zget(base + (size_t)(q / L) * nyh + q % L) : make_double2(0., 0.);
   __syncthreads();
   for (int m = threadIdx.x; m < nz; m += blockDim.x) {
-    double re = 0., im = 0.;
+    double re[L] = {}, im[L] = {};
     int q = 0;   // k m mod nz
     for (int k = 0; k < nz; k++) {
-      const double2 w = ps.tw_z[q];
+      const double2 w = tw[q];
       const double wy = SIGN < 0 ? w.y : -w.y;
-      re += col[k].x * w.x - col[k].y * wy;
-      im += col[k].x * wy + col[k].y * w.x;
+#pragma unroll
+      for (int l = 0; l < L; l++) {
+        const double2 x = col[k * L + l];
+        re[l] += x.x * w.x - x.y * wy;
+        im[l] += x.x * wy + x.y * w.x;
+      }
       q += m;
       if (q >= nz) q -= nz;
     }
-    zput(base + (size_t)m * nyh, make_double2(re, im));
+#pragma unroll
+    for (int l = 0; l < L; l++)
+      if (ky0 + l < nyh) zput(base + (size_t)m * nyh + l, make_double2(re[l], im[l]));
   }
 }
 
-// c2r transform along y of one (i, k) line into psi with its Neumann x ghosts
-// and periodic images (as iffty_kernel)
-template <class Z>
-__global__ void idfty_kernel(Geo g, Poisson ps, double * __restrict__ psi) {
-  extern __shared__ double2 spec_line[];
+// c2r transforms along y of the lines (i0 .. i0 + L - 1, k) into psi with its
+// Neumann x ghosts and periodic images (as iffty_kernel)
+template <int L, class Z>
+__global__ void __launch_bounds__(128) idfty_kernel(Geo g, Poisson ps, double * __restrict__ psi) {
+  extern __shared__ double2 tw[];
   const int ny = g.ny, nx = g.nx, nz = g.nz, nyh = ps.nyh, half = ny / 2;
-  const int i = blockIdx.x + 1, k = blockIdx.y + 1;
-  const Z * in = static_cast<const Z *>(ps.spec) + ((size_t)(i - 1) * nz + (k - 1)) * nyh;
-  for (int m = threadIdx.x; m < nyh; m += blockDim.x) {
-    double2 x = zget(in + m);
+  const int i0 = blockIdx.x * L + 1, k = blockIdx.y + 1;
+  double2 * const spec = tw + ny;   // [m][line]
+  const Z * const in = static_cast<const Z *>(ps.spec) + ((size_t)(i0 - 1) * nz + (k - 1)) * nyh;
+  for (int j = threadIdx.x; j < ny; j += blockDim.x) tw[j] = ps.tw_y[j];
+  for (int q = threadIdx.x; q < nyh * L; q += blockDim.x) {
+    const int l = q / nyh, m = q % nyh;
+    double2 x = i0 + l <= nx ? zget(in + (size_t)l * nz * nyh + m) : make_double2(0., 0.);
     if (m == 0 || m == half) x.y = 0.;
-    spec_line[m] = x;
+    spec[m * L + l] = x;
   }
   __syncthreads();
   for (int j = threadIdx.x; j < ny; j += blockDim.x) {
     // X_0 + (-1)^j X_{N/2} + 2 Re sum_{0 < m < N/2} X_m exp(+2 pi i j m / N)
-    double acc = 0.;
+    double acc[L] = {};
     int q = j;   // j m mod ny for m = 1
     for (int m = 1; m < half; m++) {
-      const double2 w = ps.tw_y[q];     // exp(-2 pi i q / N): conjugated below
-      acc += spec_line[m].x * w.x + spec_line[m].y * w.y;
+      const double2 w = tw[q];     // exp(-2 pi i q / N): conjugated below
+#pragma unroll
+      for (int l = 0; l < L; l++) acc[l] += spec[m * L + l].x * w.x + spec[m * L + l].y * w.y;
       q += j;
       if (q >= ny) q -= ny;
     }
-    const double val = spec_line[0].x + ((j & 1) ? -spec_line[half].x : spec_line[half].x) + 2. * acc;
-    auto put = [&](int jj, int kk) {
-      psi[cidx(g, i, jj, kk)] = val;
-      if (i == 1) psi[cidx(g, 0, jj, kk)] = val;
-      if (i == nx) psi[cidx(g, nx + 1, jj, kk)] = val;
-    };
-    put(j + 1, k);
-    for_images(j + 1, k, ny, nz, put);
+#pragma unroll
+    for (int l = 0; l < L; l++) {
+      const int i = i0 + l;
+      if (i > nx) break;
+      const double val = spec[l].x + ((j & 1) ? -spec[half * L + l].x : spec[half * L + l].x) + 2. * acc[l];
+      auto put = [&](int jj, int kk) {
+        psi[cidx(g, i, jj, kk)] = val;
+        if (i == 1) psi[cidx(g, 0, jj, kk)] = val;
+        if (i == nx) psi[cidx(g, nx + 1, jj, kk)] = val;
+      };
+      put(j + 1, k);
+      for_images(j + 1, k, ny, nz, put);
+    }
   }
+}
+
+template <class T, class Z>
+static void launch_div_dfty(const Geo & g, const Coefs & cf, const Poisson & ps, const FieldsT<T> & f,
+                            const double * dtp, int rkstep, cudaStream_t st) {
+  const int L = dft_lines(g.ny, sizeof(double), (long long)g.nx * g.nz);
+  const dim3 grid((g.nx + L - 1) / L, g.nz);
+  const size_t smem = (size_t)g.ny * (sizeof(double2) + L * sizeof(double));
+  auto k = L == 8 ? div_dfty_kernel<8, T, Z> : L == 4 ? div_dfty_kernel<4, T, Z> : L == 2 ? div_dfty_kernel<2, T, Z>
+                                                                                          : div_dfty_kernel<1, T, Z>;
+  k<<<grid, 128, smem, st>>>(g, cf, ps, f.ux, f.uy, f.uz, dtp, rkstep);
+}
+template <int SIGN, class Z>
+static void launch_dftz(const Geo & g, const Poisson & ps, cudaStream_t st) {
+  const int L = dft_lines(g.nz, sizeof(double2), (long long)ps.nyh * g.nx);
+  const dim3 grid((ps.nyh + L - 1) / L, g.nx);
+  auto k = L == 8 ? dftz_kernel<8, SIGN, Z> : L == 4 ? dftz_kernel<4, SIGN, Z> : L == 2 ? dftz_kernel<2, SIGN, Z>
+                                                                                        : dftz_kernel<1, SIGN, Z>;
+  k<<<grid, 128, (size_t)g.nz * (1 + L) * sizeof(double2), st>>>(g, ps);
+}
+template <class Z>
+static void launch_idfty(const Geo & g, const Poisson & ps, double * psi, cudaStream_t st) {
+  const int L = dft_lines(g.ny, sizeof(double2), (long long)g.nx * g.nz);   // a line takes 16 nyh bytes: half of this
+  const dim3 grid((g.nx + L - 1) / L, g.nz);
+  const size_t smem = sizeof(double2) * ((size_t)g.ny + (size_t)L * ps.nyh);
+  auto k = L == 8 ? idfty_kernel<8, Z> : L == 4 ? idfty_kernel<4, Z> : L == 2 ? idfty_kernel<2, Z> : idfty_kernel<1, Z>;
+  k<<<grid, 128, smem, st>>>(g, ps, psi);
 }
 
 // --------------------------------------------------------------- launchers
@@ -1245,7 +1318,6 @@ static void launch_poisson_t(const Geo & g, const Coefs & cf, const Poisson & ps
   const int tply = g.ny / EPTY;
   const size_t smy = sizeof(Z) * (size_t)Py * padded_len(g.ny);
   dim3 gy((g.nx + 2 * Py - 1) / (2 * Py), g.nz);
-  const dim3 gl(g.nx, g.nz);   // one CTA per (i, k) line of the direct transforms in y
   constexpr bool MIX = sizeof(Z) == 16;   // FP64 contexts: mixed radices; FP32-storage ones: direct sums
   const int My = mixed_lines(g.ny, (g.nx + 1) / 2), Mz = mixed_lines(g.nz, ps.nyh);
   const dim3 gmy((g.nx + 2 * My - 1) / (2 * My), g.nz), gmz((ps.nyh + Mz - 1) / Mz, g.nx);
@@ -1255,7 +1327,7 @@ static void launch_poisson_t(const Geo & g, const Coefs & cf, const Poisson & ps
   if (fy) div_ffty_kernel<EPTY, T, Z><<<gy, Py * tply, smy, st>>>(g, cf, ps, Py, lgy, f.ux, f.uy, f.uz, dtp, rkstep);
   else if constexpr (MIX)
     div_mixy_kernel<<<gmy, 256, smmy, st>>>(g, cf, ps, ry, My, f.ux, f.uy, f.uz, dtp, rkstep);
-  else div_dfty_kernel<T, Z><<<gl, 128, sizeof(double) * g.ny, st>>>(g, cf, ps, f.ux, f.uy, f.uz, dtp, rkstep);
+  else launch_div_dfty<T, Z>(g, cf, ps, f, dtp, rkstep, st);
   mark(pm.k_div);
   const int Pz = lines_per_cta(g.nz, ps.nyh, EPTZ, TC_FFTZ_THREADS);
   const int tplz = g.nz / EPTZ;
@@ -1265,10 +1337,9 @@ static void launch_poisson_t(const Geo & g, const Coefs & cf, const Poisson & ps
 #else
   dim3 gz(g.nx, (ps.nyh + Pz - 1) / Pz);
 #endif
-  const dim3 gc(ps.nyh, g.nx);   // one CTA per (ky, i) column of the direct transforms in z
   if (fz) fftz_kernel<EPTZ, -1, Z><<<gz, Pz * tplz, smz, st>>>(g, ps, Pz, lgz);
   else if constexpr (MIX) mixz_kernel<-1><<<gmz, 256, smmz, st>>>(g, ps, rz, Mz);
-  else dftz_kernel<-1, Z><<<gc, 128, sizeof(double2) * g.nz, st>>>(g, ps);
+  else launch_dftz<-1, Z>(g, ps, st);
   mark(pm.k_fwd);
   if (!launch_tdm_lines<Z>(g, ps, st)) {
     const long long nl = (long long)ps.nyh * g.nz;
@@ -1277,7 +1348,7 @@ static void launch_poisson_t(const Geo & g, const Coefs & cf, const Poisson & ps
   mark(pm.k_tdm);
   if (fz) fftz_kernel<EPTZ, +1, Z><<<gz, Pz * tplz, smz, st>>>(g, ps, Pz, lgz);
   else if constexpr (MIX) mixz_kernel<+1><<<gmz, 256, smmz, st>>>(g, ps, rz, Mz);
-  else dftz_kernel<+1, Z><<<gc, 128, sizeof(double2) * g.nz, st>>>(g, ps);
+  else launch_dftz<+1, Z>(g, ps, st);
   mark(pm.k_inv);
   constexpr bool bulk = sizeof(Z) == 16;   // staged spectrum rows need 16-byte values
   if (fy && bulk && g.ny >= 16)   // two rows of nyh values fit a padded line buffer from ny = 16 on
@@ -1285,7 +1356,7 @@ static void launch_poisson_t(const Geo & g, const Coefs & cf, const Poisson & ps
   else if (fy)
     iffty_kernel<EPTY, Z, false><<<gy, Py * tply, smy, st>>>(g, ps, Py, lgy, f.psi);
   else if constexpr (MIX) imixy_kernel<<<gmy, 256, smmy, st>>>(g, ps, ry, My, f.psi);
-  else idfty_kernel<Z><<<gl, 128, sizeof(double2) * ps.nyh, st>>>(g, ps, f.psi);
+  else launch_idfty<Z>(g, ps, f.psi, st);
   mark(pm.k_ify);
 }
 
@@ -1356,6 +1427,8 @@ void poisson_smem_limits() {
 #undef X
   allow_dyn_smem(tdm_lines_kernel<8, float2>);
   allow_dyn_smem(tdm_lines_kernel<4, float2>);
+  allow_dyn_smem(dftz_kernel<1, -1, float2>);   // the longest lines: 64 KB
+  allow_dyn_smem(dftz_kernel<1, +1, float2>);
 }
 
 }  // namespace tcgpu
