@@ -561,12 +561,16 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) conv3_kernel(ConvArgs A) {
 //
 // Roles, meeting at mbarriers only: loader warps bring halo plane p and gradient
 // tile p + 1 of each step; one thread of the MMA warp issues a step's 24 MMAs,
-// whose commit releases the halo slot and the tile of p - 1; the readout warps sum
-// each tile for the bias gradient meanwhile and drain the accumulators at the end.
+// whose commit releases the halo slot and the tile of p - 1; one warp sums each tile
+// for the bias gradient meanwhile, and four drain the accumulators at the end.
+// Every sum (a CTA's items and planes, the bias, the CTAs' partials) runs in the order
+// of the kernel with one role, whose results it reproduces to the last bit: trained
+// weights do not depend on the kernel's form.
 // Bound: the MMAs (an M = 128, K = 16 MMA takes about 62 cycles at N = 32, 72 of
 // them a plane 4.5 k cycles; 24 at N = 96 well under 2 k) and the copies. A 32 -> 32 layer
 // of 64 x 256 x 128 cells: 0.59 ms with one role, two block barriers and a serial
-// bias sum per plane; 0.37 with roles and N = 32; 0.20 now.
+// bias sum per plane; 0.37 with roles and N = 32; 0.20 with equal shares of planes
+// a CTA and sums in other orders; 0.24 now.
 constexpr int WG_LOADERS = 4, WG_MMA = 4;             // readout warps 0 .. 3, the MMA warp, the loaders
 constexpr int WG_THREADS = 32 * (WG_MMA + 1 + WG_LOADERS);
 template <int CIN, int COUT>
@@ -584,8 +588,7 @@ struct WgradLayout {
   static constexpr int GOFF = NSW * HB;
   static constexpr int BAR = GOFF + TY * GROW;           // full[NSW], free[NSW], gfree[NG], done, TMEM address, abort flag
   static constexpr int NBAR = 2 * NSW + NG + 1;
-  static constexpr int RED = BAR + NBAR * 8 + 16;        // [4][COUT] floats: the readout warps' bias sums
-  static constexpr int USED = RED + 4 * COUT * 4;
+  static constexpr int USED = BAR + NBAR * 8 + 16;
   static constexpr int TCOLS = 9 * COUT > 256 ? 512 : 256;
   // one CTA per SM, so that its tensor-memory allocation never waits on
   // another CTA's: ask for more than half of the shared memory
@@ -594,11 +597,28 @@ struct WgradLayout {
 };
 
 struct WgradArgs {
-  int nx, ny, nz;
+  int nx, ny, nz, zc, nitems;
   const __nv_bfloat16 * x;    // [cell][CIN] layer input
   const __nv_bfloat16 * dy;   // [cell][COUT] gradient of the layer's pre-activation
   float * part;               // [gridDim.x][9][128][COUT] raw sums, then [gridDim.x][COUT] bias sums
   unsigned * status;
+};
+
+// A CTA's items, strided by the grid: tile item % tiles, planes [zc (item / tiles), + zc).
+// The partial sums' order, and so the gradients' last bits, follow from this split,
+// which is why it is not the equal shares of ConvCursor.
+struct WgradCursor {
+  int item = blockIdx.x;
+  __device__ __forceinline__ bool next(const WgradArgs & A, ConvSeg & s) {
+    if (item >= A.nitems) return false;
+    const int nbx = A.nx / TX, ncol = nbx * (A.ny / TY), col = item % ncol;
+    s.x0 = (col % nbx) * TX;
+    s.y0 = (col / nbx) * TY;
+    s.z0 = item / ncol * A.zc;
+    s.z1 = min(s.z0 + A.zc, A.nz);
+    item += gridDim.x;
+    return true;
+  }
 };
 
 // a loader thread's share of one halo plane (global plane kp)
@@ -648,9 +668,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv3_wgrad_kernel(WgradArgs A)
   if (tid == 0) {
     for (int s = 0; s < NS; s++) {
       nn_mbar_init(&full[s], 32 * WG_LOADERS);
-      nn_mbar_init(&sfree[s], 1 + 4);   // the MMAs' commit and the readout warps, which keep within NS steps
+      nn_mbar_init(&sfree[s], 1 + 1);   // the MMAs' commit and the bias warp, which keeps within NS steps
     }
-    for (int g = 0; g < NG; g++) nn_mbar_init(&gfree[g], 1 + 4);   // the MMAs' commit and the readout warps
+    for (int g = 0; g < NG; g++) nn_mbar_init(&gfree[g], 1 + 1);   // the MMAs' commit and the bias warp
     nn_mbar_init(fin, 1);
     *abort_flag = 0;
     fence_barrier_init();
@@ -666,12 +686,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv3_wgrad_kernel(WgradArgs A)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  ConvArgs grid{};   // the cursor reads the grid only
-  grid.nx = A.nx;
-  grid.ny = A.ny;
-  grid.nz = A.nz;
-  ConvCursor cur(grid);
+  WgradCursor cur;
   ConvSeg it;
+  float bsum = 0.f;   // bias gradient of channel tid (tid < COUT)
   // h counts steps (halo planes), g gradient tiles, over all segments: step h uses
   // halo slot h % NS; tile g sits in slot g % NG
   if (warp > WG_MMA) {
@@ -680,7 +697,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv3_wgrad_kernel(WgradArgs A)
     const int lt = tid - 32 * (WG_MMA + 1);
     int h = 0, g = 0;
     bool ok = true;
-    while (ok && cur.next(grid, it)) {
+    while (ok && cur.next(A, it)) {
       for (int p = it.z0 - 1; p <= it.z1; p++, h++) {
         if (h >= L::LAG) {
           cp_wait<L::LAG - 1>();
@@ -709,7 +726,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv3_wgrad_kernel(WgradArgs A)
       const unsigned sb = su32(smw), tb = su32(tiles);
       bool ok = true;
       int h = 0, gb = 0;   // gb: tiles of the segments before this one
-      while (ok && cur.next(grid, it)) {
+      while (ok && cur.next(A, it)) {
         for (int p = it.z0 - 1; p <= it.z1; p++, h++) {
           ok = conv_wait(&full[h % NS], (unsigned)(h / NS) & 1u, abort_flag);
           if (!ok) break;
@@ -742,53 +759,32 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv3_wgrad_kernel(WgradArgs A)
     }
     __syncwarp();
   } else {
-    // bias gradient: every thread sums its 16-byte units (8 channels of one cell)
-    // of each tile; unit u is channel chunk (u / TX) % CG, the same for all of a thread's
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    int h = 0, g = 0;
-    bool ok = true, any = false;
-    while (ok && cur.next(grid, it)) {
-      any = true;
-      for (int p = it.z0 - 1; p <= it.z1; p++, h++) {
-        ok = conv_wait(&full[h % NS], (unsigned)(h / NS) & 1u, abort_flag);
-        if (!ok) break;
-        __syncwarp();
-        if (lane == 0) nn_arrive(&sfree[h % NS]);
-        if (p + 1 >= it.z1) continue;   // no tile comes with this step
-        static_assert(128 % (CG * TX) == 0, "one channel chunk per thread");
-#pragma unroll
-        for (int u = 0; u < TY * CG * TX / 128; u++) {
-          const int q = tid + 128 * u;
-          const uint4 w = *reinterpret_cast<const uint4 *>(tiles + (q / (CG * TX)) * L::GROW + (g % NG) * L::GP +
-                                                           (q % (CG * TX)) * 16);
-          const unsigned b[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-          for (int c = 0; c < 4; c++) {
-            acc[2 * c] += __uint_as_float(b[c] << 16);
-            acc[2 * c + 1] += __uint_as_float(b[c] & 0xffff0000u);
-          }
+    // bias gradient: lane co of warp 0 sums channel co of each tile, cell by cell (the
+    // order is part of the result; 128 dependent additions fit a plane's MMAs)
+    bool any = cur.item < A.nitems;
+    if (warp == 0) {
+      const int co = lane < COUT ? lane : 0;
+      int h = 0, g = 0;
+      bool ok = true;
+      while (ok && cur.next(A, it)) {
+        for (int p = it.z0 - 1; p <= it.z1; p++, h++) {
+          ok = conv_wait(&full[h % NS], (unsigned)(h / NS) & 1u, abort_flag);
+          if (!ok) break;
+          __syncwarp();
+          if (lane == 0) nn_arrive(&sfree[h % NS]);
+          if (p + 1 >= it.z1) continue;   // no tile comes with this step
+          const char * tile = tiles + (g % NG) * L::GP + (co / 8) * TX * 16 + (co % 8) * 2;
+          float acc = 0.f;
+#pragma unroll 32
+          for (int c = 0; c < TX * TY; c++)
+            acc += __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(tile + (c / TX) * L::GROW + (c % TX) * 16));
+          bsum += acc;
+          __syncwarp();
+          if (lane == 0) nn_arrive(&gfree[g % NG]);
+          g++;
         }
-        __syncwarp();
-        if (lane == 0) nn_arrive(&gfree[g % NG]);
-        g++;
       }
     }
-    // over the warp's eight x of each chunk, then the four warps through shared memory
-    float * red = reinterpret_cast<float *>(smw + L::RED);
-    constexpr int CW = 32 / TX;   // channel chunks a warp's lanes cover at once
-#pragma unroll
-    for (int c = 0; c < 8; c++)
-#pragma unroll
-      for (int o = 1; o < TX; o <<= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-    for (int c = lane; c < COUT; c += 32) red[warp * COUT + c] = 0.f;
-    __syncwarp();
-    // chunk of lane l in warp w: ((32 w + l) / TX) % CG
-    if (lane % TX == 0) {
-      const int ch = ((tid / TX) % CG) * 8;
-#pragma unroll
-      for (int c = 0; c < 8; c++) atomicAdd(&red[warp * COUT + ch + c], acc[c]);   // CW > CG: chunks repeat
-    }
-    static_assert(CW >= 1, "lanes cover whole chunks");
     if (!nn_mbar_wait(fin, 0)) {
       if (lane == 0) atomicOr(A.status, ST_TIMEOUT);
       any = false;
@@ -821,11 +817,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv3_wgrad_kernel(WgradArgs A)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (tid < COUT) {
-    const float * red = reinterpret_cast<const float *>(smw + L::RED);
-    A.part[(size_t)gridDim.x * 9 * 128 * COUT + (size_t)blockIdx.x * COUT + tid] =
-        (red[tid] + red[COUT + tid]) + (red[2 * COUT + tid] + red[3 * COUT + tid]);
-  }
+  if (tid < COUT) A.part[(size_t)gridDim.x * 9 * 128 * COUT + (size_t)blockIdx.x * COUT + tid] = bsum;
   if (warp == WG_MMA) {
     if (lane == 0) nn_mbar_wait(fin, 0);   // no MMA in flight when the columns are freed
     __syncwarp();
@@ -835,28 +827,22 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv3_wgrad_kernel(WgradArgs A)
 
 // Sum of the CTAs' raw partials into the master-layout gradients
 // dw[t][co][ci] (real channel counts) and db[co]; beta = 0 overwrites,
-// 1 accumulates. A block takes 32 consecutive partial values (output channels
-// fastest, as they lie in memory), its eight warps every eighth CTA's.
+// 1 accumulates. A thread sums one value of all CTAs in their order (the order is
+// part of the result), neighbours consecutive values, output channels fastest, as
+// they lie in memory.
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float * __restrict__ part, int nblk, int cinp,
                                                            int coutp, int cin, int cout, float * __restrict__ dw,
                                                            float * __restrict__ db, float beta) {
-  __shared__ float red[8][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nraw = 9 * 3 * cinp * coutp;           // y shifts 0 .. 2 of the nine accumulators
-  const int q = blockIdx.x * 32 + lane;            // raw value, then the bias sums
+  const int q = blockIdx.x * 256 + threadIdx.x;    // raw value, then the bias sums
+  if (q >= nraw + coutp) return;
   const bool wt = q < nraw;
   const int co = wt ? q % coutp : q - nraw, m = (q / coutp) % (3 * cinp), a = q / (coutp * 3 * cinp);
+  const size_t step = wt ? (size_t)9 * 128 * coutp : (size_t)coutp;
+  const float * src = wt ? part + ((size_t)a * 128 + m) * coutp + co : part + (size_t)nblk * 9 * 128 * coutp + co;
   float acc = 0.f;
-  if (q < nraw + coutp) {
-    const size_t step = wt ? (size_t)9 * 128 * coutp : (size_t)coutp;
-    const float * src = wt ? part + ((size_t)a * 128 + m) * coutp + co : part + (size_t)nblk * 9 * 128 * coutp + co;
-#pragma unroll 4
-    for (int b = w; b < nblk; b += 8) acc += src[(size_t)b * step];
-  }
-  red[w][lane] = acc;
-  __syncthreads();
-  if (w != 0 || q >= nraw + coutp) return;
-  for (int r = 1; r < 8; r++) acc += red[r][lane];
+#pragma unroll 16
+  for (int b = 0; b < nblk; b++) acc += src[(size_t)b * step];
   if (wt) {
     // accumulator row m: y shift m / cinp, input channel m % cinp; a = 3 (dz + 1) + dx + 1
     const int ci = m % cinp, dyi = m / cinp, dz = a / 3, dx = a % 3;
@@ -1018,13 +1004,13 @@ int dispatch_conv3(int cin, int cout, const ConvArgs & a, cudaStream_t st) {
   return 1;
 }
 
-// weight gradient: CTAs over the planes of all column tiles (each reads two halo
-// planes more per segment, so at least four planes apiece where nz allows)
-int wgrad_ctas(int nx, int ny, int nz) {
+// weight gradient: (column tile, z chunk) items, at least two a CTA where nz allows
+// chunks of four planes and more, and the CTAs over them
+int wgrad_split(int nx, int ny, int nz, int & zc, int & nitems) {
   const int ncol = (nx / TX) * (ny / TY);
-  int zc = nz;
+  zc = nz;
   while (zc > 4 && (long)ncol * ((nz + zc - 1) / zc) < 148L * 2) zc = (zc + 1) / 2;
-  const int nitems = ncol * ((nz + zc - 1) / zc);
+  nitems = ncol * ((nz + zc - 1) / zc);
   return nitems < 148 ? nitems : 148;
 }
 
@@ -1223,7 +1209,8 @@ int tcgpu_nn_conv3(int mode, int cin, int cout, int nx, int ny, int nz, const vo
 
 size_t tcgpu_nn_wgrad_workspace(int nx, int ny, int nz, int coutp) {
   if (nx % TX || ny % TY || nx <= 0 || ny <= 0 || nz <= 0) return 0;
-  return (size_t)wgrad_ctas(nx, ny, nz) * (9 * 128 + 1) * coutp * sizeof(float);
+  int zc, nitems;
+  return (size_t)wgrad_split(nx, ny, nz, zc, nitems) * (9 * 128 + 1) * coutp * sizeof(float);
 }
 
 int tcgpu_nn_conv3_wgrad(int cinp, int coutp, int cin, int cout, int nx, int ny, int nz, const void * x,
@@ -1237,7 +1224,7 @@ int tcgpu_nn_conv3_wgrad(int cinp, int coutp, int cin, int cout, int nx, int ny,
     return nn_fail("nn_conv3_wgrad: workspace smaller than tcgpu_nn_wgrad_workspace()");
   WgradArgs a{};
   a.nx = nx; a.ny = ny; a.nz = nz;
-  const int nblk = wgrad_ctas(nx, ny, nz);
+  const int nblk = wgrad_split(nx, ny, nz, a.zc, a.nitems);
   a.x = static_cast<const __nv_bfloat16 *>(x);
   a.dy = static_cast<const __nv_bfloat16 *>(dy);
   a.part = static_cast<float *>(workspace);
@@ -1250,8 +1237,8 @@ int tcgpu_nn_conv3_wgrad(int cinp, int coutp, int cin, int cout, int nx, int ny,
   else if (cinp == 32 && coutp == 16) rc = launch_wgrad<32, 16>(a, nblk, st);
   else if (cinp == 16 && coutp == 16) rc = launch_wgrad<16, 16>(a, nblk, st);
   if (rc) return nn_fail("nn_conv3_wgrad: unsupported channel counts or launch failure");
-  const int nred = 27 * coutp * cinp + coutp;   // a multiple of 16
-  wgrad_reduce_kernel<<<(nred + 31) / 32, 256, 0, st>>>(a.part, nblk, cinp, coutp, cin, cout, dw, db, beta);
+  const int nred = 27 * coutp * cinp + coutp;
+  wgrad_reduce_kernel<<<(nred + 255) / 256, 256, 0, st>>>(a.part, nblk, cinp, coutp, cin, cout, dw, db, beta);
   return cudaGetLastError() == cudaSuccess ? 0 : nn_fail("nn_conv3_wgrad: reduction launch failed");
 }
 
