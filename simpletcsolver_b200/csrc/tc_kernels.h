@@ -303,7 +303,7 @@ void launch_tensors(const Geo & g, const Coefs & cf, const FieldBufs & f, const 
 // logging reductions (src/logging/*.c); out: 9 doubles on the device,
 // partial: DIAG_BLOCKS x 9 doubles of scratch; f: current fields, fs: the
 // fields the momentum injection / dissipation tensors are formed from
-constexpr int DIAG_BLOCKS_MAX = 296;
+constexpr int DIAG_BLOCKS_MAX = 444;
 void launch_diagnostics(const Geo & g, const Coefs & cf, const Bc & bc, const FieldBufs & f, const FieldBufs & fs,
                         double nu, double kappa, double * out, double * partial, cudaStream_t st);
 

@@ -466,7 +466,7 @@ void launch_tensors(const Geo & g, const Coefs & cf, const FieldBufs & f, const 
 
 // --------------------------------------------------------------- diagnostics
 // partial[b][0..8]: max|div|, inj_m, inj_s, dis_m, dis_s, e_ux, e_uy, e_uz, e_t
-constexpr int DIAG_BLOCKS = 296;
+constexpr int DIAG_BLOCKS = 444;
 
 // f: the current fields (divergence, energies, the wall velocity of the
 // momentum injection, every scalar term); fs: the fields the velocity-gradient
@@ -474,11 +474,17 @@ constexpr int DIAG_BLOCKS = 296;
 // reference logs tensors of the last predict's input fields
 // (src/fluid/predict/main.c:56-82, read by src/logging/injection.c:49-51 and
 // dissipation.c); fs = f gives the tensors of the current fields.
+// A warp takes whole radial lines, a lane every 32nd face; lengths divide as
+// tabulated reciprocals.
+// Bound: shared by the L1 (about 40 reads a cell, most of them neighbours') and the
+// FP64 pipe; HBM needs 32 bytes a cell (56 with the gradients of other fields). With a
+// 64-bit division for each cell's indices, four FP64 divisions a cell and one thread
+// per sum at the end: 84 + 38 us at 64 x 256 x 128, 70 + 5 here.
 template <class T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 diag_kernel(Geo g, Coefs cf, Bc bc, FieldsT<T> f, FieldsT<T> fs, double * partial) {
   const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const long long total = (long long)(nx + 1) * ny * nz;
+  const int lines = ny * nz, warp = blockIdx.x * 8 + (threadIdx.x >> 5);
   double acc[9] = {0., 0., 0., 0., 0., 0., 0., 0., 0.};
   const T * ux = f.ux;
   const T * uy = f.uy;
@@ -487,14 +493,10 @@ diag_kernel(Geo g, Coefs cf, Bc bc, FieldsT<T> f, FieldsT<T> fs, double * partia
   const T * sux = fs.ux;
   const T * suy = fs.uy;
   const T * suz = fs.uz;
-  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < total;
-       c += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(c % (nx + 1)) + 1;     // 1..nx+1
-    const long long r = c / (nx + 1);
-    const int j = (int)(r % ny) + 1;
-    const int k = (int)(r / ny) + 1;
+  for (int r = warp; r < lines; r += gridDim.x * 8)
+  for (int i = (threadIdx.x & 31) + 1; i <= nx + 1; i += 32) {
+    const int j = r % ny + 1, k = r / ny + 1;
     const double jdf = __ldg(g.jdxf + i);
-    const double hxf = __ldg(g.hxxf + i);
     // face quantities at i
     const double ih = __ldg(cf.c_invhxxf + i);
     const double uyim = (double)uy[sidx_c<T>(g, i - 1, j, k)], uyi = (double)uy[sidx_c<T>(g, i, j, k)];
@@ -511,18 +513,18 @@ diag_kernel(Geo g, Coefs cf, Bc bc, FieldsT<T> f, FieldsT<T> fs, double * partia
     acc[3] += jdf * lxz * (lxz + lzx);
     {  // dissipation.c:240-265 (scalar, x)
       const double d = -(double)t[sidx_c<T>(g, i - 1, j, k)] + (double)t[sidx_c<T>(g, i, j, k)];
-      const double q = d / hxf;
+      const double q = d * ih;
       acc[4] += jdf * (q * q);
     }
     // injection.c:55-98 at the two walls
     if (i == 1 || i == nx + 1) {
       const double sgn = (i == 1) ? -1. : 1.;
       const double uyw = (i == 1) ? uyim : uyi;
-      acc[1] += sgn * jdf / hxf * uyw * (lyx + lxy);
+      acc[1] += sgn * jdf * ih * uyw * (lyx + lxy);
       const double tw = (i == 1) ? (double)t[sidx_c<T>(g, 0, j, k)] : (double)t[sidx_c<T>(g, nx + 1, j, k)];
       const double dtw = (i == 1) ? (-(double)t[sidx_c<T>(g, 0, j, k)] + (double)t[sidx_c<T>(g, 1, j, k)])
                                   : (-(double)t[sidx_c<T>(g, nx, j, k)] + (double)t[sidx_c<T>(g, nx + 1, j, k)]);
-      acc[2] += sgn * jdf / hxf * tw / hxf * dtw;
+      acc[2] += sgn * jdf * ih * tw * ih * dtw;
     }
     if (i >= 2 && i <= nx) {  // total_energy.c:45-51
       const double v = (double)ux[sidx_f<T>(g, i, j, k)];
@@ -556,11 +558,11 @@ diag_kernel(Geo g, Coefs cf, Bc bc, FieldsT<T> f, FieldsT<T> fs, double * partia
       acc[3] += jdc * lzz * (lzz + lzz);
       const double t0 = (double)t[sidx_c<T>(g, i, j, k)];
       {
-        const double q = (-(double)t[sidx_c<T>(g, i, j - 1, k)] + t0) / __ldg(g.hyxc + i);
+        const double q = (-(double)t[sidx_c<T>(g, i, j - 1, k)] + t0) * ihy;
         acc[4] += jdc * (q * q);
       }
       {
-        const double q = (-(double)t[sidx_c<T>(g, i, j, k - 1)] + t0) / g.hz;
+        const double q = (-(double)t[sidx_c<T>(g, i, j, k - 1)] + t0) * cf.inv_hz;
         acc[4] += jdc * (q * q);
       }
       acc[6] += jdc * 0.5 * (uy0 * uy0);
@@ -587,21 +589,29 @@ diag_kernel(Geo g, Coefs cf, Bc bc, FieldsT<T> f, FieldsT<T> fs, double * partia
   }
 }
 
-__global__ void diag_final_kernel(const double * partial, int nblocks, double nu, double kappa, double * out) {
-  const int q = threadIdx.x;
-  if (q >= 9) return;
-  double v = partial[q];
-  for (int b = 1; b < nblocks; b++) v = (q == 0) ? fmax(v, partial[(size_t)b * 9 + q]) : v + partial[(size_t)b * 9 + q];
+// one warp per quantity
+__global__ void __launch_bounds__(288) diag_final_kernel(const double * partial, int nblocks, double nu, double kappa,
+                                                         double * out) {
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double v = 0.;
+  for (int b = lane; b < nblocks; b += 32) {
+    const double w = partial[(size_t)b * 9 + q];
+    v = (q == 0) ? fmax(v, w) : v + w;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const double w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = (q == 0) ? fmax(v, w) : v + w;
+  }
   if (q == 1 || q == 3) v *= nu;
   if (q == 2 || q == 4) v *= kappa;
-  out[q] = v;
+  if (lane == 0) out[q] = v;
 }
 
 void launch_diagnostics(const Geo & g, const Coefs & cf, const Bc & bc, const FieldBufs & f, const FieldBufs & fs,
                         double nu, double kappa, double * out, double * partial, cudaStream_t st) {
   if (f.bytes == 4) diag_kernel<float><<<DIAG_BLOCKS, 256, 0, st>>>(g, cf, bc, f.as<float>(), fs.as<float>(), partial);
   else diag_kernel<double><<<DIAG_BLOCKS, 256, 0, st>>>(g, cf, bc, f.as<double>(), fs.as<double>(), partial);
-  diag_final_kernel<<<1, 32, 0, st>>>(partial, DIAG_BLOCKS, nu, kappa, out);
+  diag_final_kernel<<<1, 288, 0, st>>>(partial, DIAG_BLOCKS, nu, kappa, out);
 }
 
 // --------------------------------------------------------------- statistics
