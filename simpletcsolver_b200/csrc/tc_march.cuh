@@ -13,22 +13,27 @@
 // holds the rows j0-1 .. j0+JT of ux, uy, uz, t and j0-1 .. j0+JT-1 of p; the
 // previous substep's source terms of the CTA's lines arrive in a two-plane
 // buffer of their own. Roles, which meet only at mbarriers:
-//   group A (NW PAIRS warps)  ux at face i and t at centre i of a line pair
-//   group B (NW PAIRS warps)  uy and uz at centre i of a line pair
-//   solve warps (4)           variable v of every line: radial solve, update,
-//                             stores of the new fields (or of the increments),
-//                             and its copies into the ring and the old terms
-// The field groups hand a plane's increments to the solve warps through a
+//   field warps (NFW)  group A: ux at face i and t at centre i of a line pair,
+//                      group B: uy and uz at centre i; a warp has one group
+//                      (NG = 2) or both (NG = 1)
+//   solve warps (4)    variable v of every line: radial solve, update, stores of
+//                      the new fields (or of the increments), and its copies
+//                      into the ring and the old terms
+// The field warps hand a plane's increments to the solve warps through a
 // double-buffered staging area and never wait for the solutions.
 //
-// What bounds it: instruction issue. The kernel moves 104 / 136 bytes a cell
-// (the first / later substeps), 2.2 / 2.8 ms at 256 x 1024 x 512 at the copy
-// bandwidth, and its FP64 instructions need about 1.2 ms of the FP64 pipe. A
-// single field group with all four variables needs 200 registers a thread (82
-// of them coefficients) and leaves two field warps per scheduler, too few to
-// cover the fixed FP64 and shared-memory latencies; two groups of 96 registers
-// make it four, and the solve warps' stores take the wait for the solutions
-// off the field warps.
+// What bounds it: the solve warps' serial chain, with the field warps close
+// behind. The kernel moves 104 / 136 bytes a cell (the first / later substeps),
+// 2.2 / 2.8 ms at 256 x 1024 x 512 at the copy bandwidth, and its FP64 instructions
+// need about 1.2 ms of the FP64 pipe; at nx = 256 a plane of two lines takes a
+// solve warp about 4.6 thousand cycles: 2.1 the two solves (dependent FP64 and
+// shuffle latencies), 0.65 issuing copies, 0.55 the update, 0.36 the stores, the
+// rest waits. One CTA of 12 warps fits an SM: 8 field warps with both groups at
+// 176 registers and 4 solve warps at 152, none spilling. 16 field warps at 96
+// registers spill and are slower (1.80 against 1.09 ms at 256 x 512 x 256), as are
+// solves whose scans run half as far (30.7 against 27.1 ps a cell). Per launch
+// 6.8 -> 3.8 ms at 256 x 1024 x 512 against the form whose field warps solved,
+// updated and stored.
 //
 // Every face between two cells of a thread is formed once: the thread carries
 // the z face's share of the next plane's cell in registers (so plane k - 1 is
@@ -51,6 +56,7 @@ namespace tcgpu {
 namespace march {
 
 #define LD(p) __ldg(p)
+__device__ __forceinline__ void prefetch_l1(const void * p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 // Shared memory, in bytes, shared by the kernel and its launcher. Row buffers
 // are sized for the widest radial line of the warp count (nx <= 32 NW), so
@@ -712,6 +718,13 @@ struct Group {
       for (int l = 0; l < 2; l++) {
         if (acta) ea[l] += (C)fa[(size_t)l * la + step * sa];
         if (GRP == 1 && act) eb[l] += (C)fb[(size_t)l * lc + step * sb];
+      }
+      if (step + 1 < A.KC) {   // the next plane's forces into the L1 (held in registers they spill)
+#pragma unroll
+        for (int l = 0; l < 2; l++) {
+          if (acta) prefetch_l1(fa + (size_t)l * la + (step + 1) * sa);
+          if (GRP == 1 && act) prefetch_l1(fb + (size_t)l * lc + (step + 1) * sb);
+        }
       }
     }
     if (!TILE && A.rkstep != 0) {
