@@ -565,7 +565,7 @@ static int check_domain(const domain_t * d) {
   const size_t nx = d->glsizes[0], ny = d->glsizes[1], nz = d->glsizes[2];
   if (nx < 2 || nx > 1024) return fail("nx = %zu outside the supported range [2, 1024]", nx);
   // any even ny and any nz that is a multiple of 4 (powers of two take the
-  // FFT kernels, other lengths direct transforms)
+  // FFT kernels, other lengths mixed radices or direct sums)
   if (ny < 4 || ny > 2048 || ny % 2 || nz < 4 || nz > 2048 || nz % 4)
     return fail("ny = %zu must be even and nz = %zu a multiple of 4, both in [4, 2048]", ny, nz);
   if (!d->hxxf || !d->hxxc || !d->hyxf || !d->hyxc || !d->jdxf || !d->jdxc)

@@ -1312,7 +1312,7 @@ static void launch_poisson_t(const Geo & g, const Coefs & cf, const Poisson & ps
                              const double * tab_y, const double * tab_z, const double * base,
                              const double * dtp, int rkstep, cudaStream_t st, const PoissonMarks & pm) {
   auto mark = [&](int kk) { if (pm.mark) pm.mark(kk, 1); };
-  const bool fy = pow2(g.ny), fz = pow2(g.nz);   // FFTs; otherwise the direct transforms
+  const bool fy = pow2(g.ny), fz = pow2(g.nz);   // FFTs; otherwise mixed radices or direct sums
   const int lgy = ilog2(g.ny), lgz = ilog2(g.nz);
   const int Py = lines_per_cta(g.ny, (g.nx + 1) / 2, EPTY, TC_FFTY_THREADS);
   const int tply = g.ny / EPTY;
