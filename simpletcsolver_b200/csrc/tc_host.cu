@@ -123,20 +123,23 @@ struct Ctx {
 static std::map<const fluid_t *, Ctx *> g_ctx;
 static int g_storage_bytes = 8;   // storage of contexts created from now on
 
+// Device memory of a context, zero to begin with: zeroed on the context's own
+// stream, which does not wait for the legacy stream, so that every kernel and copy
+// of the context comes after the zeros whatever else the process has queued.
 static void * valloc(Ctx & c, size_t bytes) {
   void * p = nullptr;
   if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
-  cudaMemset(p, 0, bytes);
   c.allocs.push_back(p);
-  return p;
+  return cudaMemsetAsync(p, 0, bytes, c.st) == cudaSuccess ? p : nullptr;
 }
 
-static double * dalloc(Ctx & c, size_t n) {
-  void * p = nullptr;
-  if (cudaMalloc(&p, n * sizeof(double)) != cudaSuccess) return nullptr;
-  cudaMemset(p, 0, n * sizeof(double));
-  c.allocs.push_back(p);
-  return static_cast<double *>(p);
+static double * dalloc(Ctx & c, size_t n) { return static_cast<double *>(valloc(c, n * sizeof(double))); }
+
+// host values into a context's memory, in order with its stream; the host's copy
+// may go on return
+static cudaError_t upload(Ctx & c, void * dst, const void * src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c.st);
+  return e == cudaSuccess ? cudaStreamSynchronize(c.st) : e;
 }
 
 static void destroy_ctx(Ctx * c) {
@@ -201,7 +204,7 @@ static int set_physics(Ctx & c, const fluid_t * fl, const domain_t * d) {
     const double v = c.coef_dif / diffusivity * 0.5 / 3 * pow(gs[dim], 2.);
     c.caps_h[dim] = c.bc.implicit[dim] ? 0. : v;
   }
-  CK(cudaMemcpy(c.dt_caps, c.caps_h, sizeof(c.caps_h), cudaMemcpyHostToDevice));
+  CK(upload(c, c.dt_caps, c.caps_h, sizeof(c.caps_h)));
   for (int b = 0; b < 2; b++) {
     if (c.step_graph[b]) {
       cudaGraphExecDestroy(c.step_graph[b]);
@@ -345,7 +348,7 @@ static int build_tables(Ctx & c, const domain_t * d) {
   }
   double * dT = dalloc(c, T.size());
   if (!dT) return fail("cudaMalloc of coefficient tables failed");
-  CK(cudaMemcpy(dT, T.data(), T.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CK(upload(c, dT, T.data(), T.size() * sizeof(double)));
   const double * cols[NCOL];
   for (int n = 0; n < NCOL; n++) cols[n] = dT + (size_t)n * CSTRIDE;
   Coefs & cf = c.cf;
@@ -378,7 +381,7 @@ static int build_tables(Ctx & c, const domain_t * d) {
   }
   double * dG = dalloc(c, G.size());
   if (!dG) return fail("cudaMalloc failed");
-  CK(cudaMemcpy(dG, G.data(), G.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CK(upload(c, dG, G.data(), G.size() * sizeof(double)));
   c.g.nx = nx;
   c.g.ny = ny;
   c.g.nz = nz;
@@ -409,7 +412,7 @@ static int build_tables(Ctx & c, const domain_t * d) {
   }
   double * dP = dalloc(c, P.size());
   if (!dP) return fail("cudaMalloc failed");
-  CK(cudaMemcpy(dP, P.data(), P.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CK(upload(c, dP, P.data(), P.size() * sizeof(double)));
   c.xf.single = c.sb == 4;
   c.xf.ne = c.xf.single ? predict_warps32(nx) : predict_warps(nx);
   const size_t LX = (size_t)32 * c.xf.ne;   // every element a solving warp touches
@@ -493,11 +496,11 @@ static int build_tables(Ctx & c, const domain_t * d) {
   c.tab_z = dalloc(c, nz);
   c.tab_y = dalloc(c, (size_t)nx * nyh);
   if (!dtl || !dtu || !c.base || !c.tab_z || !c.tab_y) return fail("cudaMalloc failed");
-  CK(cudaMemcpy(dtl, tl.data(), nx * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(dtu, tu.data(), nx * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c.base, base.data(), nx * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c.tab_z, tz.data(), nz * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c.tab_y, ty.data(), ty.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CK(upload(c, dtl, tl.data(), nx * sizeof(double)));
+  CK(upload(c, dtu, tu.data(), nx * sizeof(double)));
+  CK(upload(c, c.base, base.data(), nx * sizeof(double)));
+  CK(upload(c, c.tab_z, tz.data(), nz * sizeof(double)));
+  CK(upload(c, c.tab_y, ty.data(), ty.size() * sizeof(double)));
   c.ps.tl = dtl;
   c.ps.tu = dtu;
   // twiddles exp(-2 pi i m / N), m < N, from libm
@@ -509,7 +512,7 @@ static int build_tables(Ctx & c, const domain_t * d) {
       tw[2 * k + 1] = -sin(a);
     }
     double * p = dalloc(c, 2 * (size_t)N);
-    if (p) cudaMemcpy(p, tw.data(), 2 * (size_t)N * sizeof(double), cudaMemcpyHostToDevice);
+    if (p && upload(c, p, tw.data(), 2 * (size_t)N * sizeof(double)) != cudaSuccess) p = nullptr;
     return reinterpret_cast<double2 *>(p);
   };
   c.ps.tw_y = twiddles(ny);
@@ -523,7 +526,7 @@ static int build_tables(Ctx & c, const domain_t * d) {
       tw[2 * k + 1] = (float)-sin(a);
     }
     float * p = static_cast<float *>(valloc(c, 2 * (size_t)N * sizeof(float)));
-    if (p) cudaMemcpy(p, tw.data(), 2 * (size_t)N * sizeof(float), cudaMemcpyHostToDevice);
+    if (p && upload(c, p, tw.data(), 2 * (size_t)N * sizeof(float)) != cudaSuccess) p = nullptr;
     return reinterpret_cast<float2 *>(p);
   };
   if (c.sb == 4) {
@@ -658,7 +661,7 @@ static Ctx * create_ctx(const domain_t * d, const fluid_t * fl) {
   c->diag_part = dalloc(*c, (size_t)DIAG_BLOCKS_MAX * 9);
   if (!c->dt_caps || !c->dtp || !c->dtmin || !c->status || !c->diag_out || !c->diag_part) return bad("cudaMalloc failed");
   const std::vector<unsigned long long> ones(DT_SLOTS, 0x3ff0000000000000ull);   // 1.0
-  if (cudaMemcpy(c->dtmin, ones.data(), DT_SLOTS * sizeof(ones[0]), cudaMemcpyHostToDevice) != cudaSuccess)
+  if (upload(*c, c->dtmin, ones.data(), DT_SLOTS * sizeof(ones[0])) != cudaSuccess)
     return bad("cudaMemcpy failed");
   if (cudaMallocHost(&c->h_scalar, 64 * sizeof(double)) != cudaSuccess) return bad("cudaMallocHost failed");
   if (cudaMallocHost(&c->h_status, sizeof(unsigned) * 4) != cudaSuccess) return bad("cudaMallocHost failed");
