@@ -576,23 +576,9 @@ static int check_domain(const domain_t * d) {
   return 0;
 }
 
-// the kernels' shared-memory limits, once per device (attributes of the kernels,
-// not of a context)
-static void allow_smem() {
-  static std::mutex m;
-  static std::vector<int> done;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return;
-  std::lock_guard<std::mutex> lk(m);
-  if (std::find(done.begin(), done.end(), dev) != done.end()) return;
-  poisson_smem_limits();
-  allow_lines_smem();
-  allow_periodic_lines_smem();
-  done.push_back(dev);
-}
-
 static Ctx * create_ctx(const domain_t * d, const fluid_t * fl) {
   if (check_domain(d)) return nullptr;
+  cudaGetLastError();   // an earlier call's error is not this context's
   Ctx * c = new Ctx();
   c->key = fl;
   c->nx = (int)d->glsizes[0];
@@ -666,7 +652,17 @@ static Ctx * create_ctx(const domain_t * d, const fluid_t * fl) {
   if (cudaMallocHost(&c->h_scalar, 64 * sizeof(double)) != cudaSuccess) return bad("cudaMallocHost failed");
   if (cudaMallocHost(&c->h_status, sizeof(unsigned) * 4) != cudaSuccess) return bad("cudaMallocHost failed");
   if (build_tables(*c, d)) { destroy_ctx(c); return nullptr; }
-  allow_smem();
+  // The kernels' shared-memory limits (those of the predict: launch_one) belong to the
+  // current CUDA context and go with it, so every device context sets them: one that
+  // relied on an earlier one's would fail after cudaDeviceReset or in another context.
+  poisson_smem_limits();
+  allow_lines_smem();
+  allow_periodic_lines_smem();
+  if (const cudaError_t e = cudaGetLastError()) {
+    fail("setting the kernels' shared-memory limits failed: %s", cudaGetErrorString(e));
+    destroy_ctx(c);
+    return nullptr;
+  }
   c->nu = 0.;
   if (set_physics(*c, fl, d)) { destroy_ctx(c); return nullptr; }
   return c;
@@ -812,19 +808,26 @@ static int launch_step(Ctx & c) {
   if (!c.dt_ready) enqueue_dtmin(c);
   const int p = c.cur;
   if (c.step_graph[p] == nullptr) {
-    cudaGraph_t graph;
+    cudaGraph_t graph = nullptr;
     Recorder count;
     Recorder * prev = g_rec;
-    g_rec = &count;
     CK(cudaStreamBeginCapture(c.st, cudaStreamCaptureModeThreadLocal));
+    g_rec = &count;
     enqueue_step(c);
-    CK(cudaStreamEndCapture(c.st, &graph));
+    cudaError_t e = cudaStreamEndCapture(c.st, &graph);
     g_rec = prev;
     c.cur = p;   // capture only recorded the launches
-    for (int k = 0; k < TCGPU_K_COUNT; k++) c.graph_launches[k] = count.launches[k];
-    cudaError_t e = cudaGraphInstantiate(&c.step_graph[p], graph, 0);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) return fail("cudaGraphInstantiate failed: %s", cudaGetErrorString(e));
+    const cudaError_t launch = cudaGetLastError();   // a launch that failed is not in the graph
+    if (e == cudaSuccess) e = launch;
+    if (e == cudaSuccess) {
+      for (int k = 0; k < TCGPU_K_COUNT; k++) c.graph_launches[k] = count.launches[k];
+      e = cudaGraphInstantiate(&c.step_graph[p], graph, 0);
+    }
+    if (graph) cudaGraphDestroy(graph);
+    if (e != cudaSuccess) {
+      c.step_graph[p] = nullptr;
+      return fail("capture of the time step failed: %s", cudaGetErrorString(e));
+    }
   }
   CK(cudaGraphLaunch(c.step_graph[p], c.st));
   c.cur = p ^ 1;   // three predicts per step: the state ends in the other buffer

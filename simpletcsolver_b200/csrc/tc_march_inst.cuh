@@ -1,7 +1,5 @@
 // Definitions behind tc_march_launch.cuh, for the instantiating files.
 #pragma once
-#include <atomic>
-
 #include "tc_march_f32.cuh"
 #include "tc_march_launch.cuh"
 
@@ -14,14 +12,10 @@ void launch_one(Args<T> A, const double * dtp, cudaStream_t st) {
   const long long columns = (long long)((A.g.ny + L::JT - 1) / L::JT) * (TILE ? (A.g.nx + L::NT - 1) / L::NT : 1);
   A.KC = march_planes(columns, A.g.nz, 1);
   auto kernel = predict_kernel<NW, PAIRS, NG, IMPL, T, TILE>;
-  static std::atomic<unsigned> allowed{0};   // devices (bit) that know this instance's shared memory
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const unsigned bit = 1u << (dev & 31);
-  if (!(allowed.load(std::memory_order_relaxed) & bit)) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES) != cudaSuccess) return;
-    allowed.fetch_or(bit, std::memory_order_relaxed);
-  }
+  // the limit belongs to the current CUDA context, so it is set with every launch (steps
+  // replay a graph: twice per device context); a failure stays the thread's last error,
+  // which the capture of a step and the end of each entry point report
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES) != cudaSuccess) return;
   kernel<<<(unsigned)(columns * (A.g.nz / A.KC)), L::THREADS, L::BYTES, st>>>(A, dtp);
 }
 

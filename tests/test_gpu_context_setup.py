@@ -1,5 +1,9 @@
-"""Device contexts set up while the process is busy elsewhere on the GPU: nothing of a
-context may depend on the legacy default stream, which its own stream does not wait for."""
+"""Device contexts set up while the process is busy elsewhere on the GPU (nothing of a
+context may depend on the legacy default stream, which its own stream does not wait for),
+and in one CUDA context after another."""
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -7,6 +11,8 @@ import pytest
 
 from simpletcsolver_b200 import abi, ic
 from simpletcsolver_b200.solver import Solver
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +58,51 @@ def test_set_up_beside_a_busy_default_stream(lib, tmp_path, nx, ny, nz, storage)
         torch.cuda.synchronize()
     for w, g in zip(want, got):
         assert np.isfinite(g).all() and np.array_equal(w, g)   # the same kernels on the same values
+
+
+CHILD = """
+import ctypes as C, dataclasses, sys, tempfile
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+from simpletcsolver_b200 import abi, ic
+from simpletcsolver_b200.solver import Solver
+
+cu, lib = C.CDLL("libcuda.so.1"), abi.load()
+
+def ok(status):
+    assert status == 0, status
+
+def steps():
+    out = []
+    for make, n, implicit, storage in ((ic.taylor_couette, (64, 16, 16), "x", 8), (ic.taylor_couette, (256, 12, 20), "x", 8),
+                                       (ic.plane_couette, (320, 32, 16), "xyz", 8), (ic.taylor_couette, (96, 16, 16), "x", 4)):
+        case = dataclasses.replace(make(*n, 500.0), implicit=tuple(d in implicit for d in "xyz"))
+        with tempfile.TemporaryDirectory() as d:
+            s = Solver.from_case(case, d, lib=lib, coherence=abi.NO_COHERENCE, storage=storage)
+        out.append(s.run(3))
+        s.pull()
+        out += [s.field(f).copy() for f in ("ux", "uy", "uz", "p", "t")]
+        s.release()
+    return out
+
+ok(cu.cuInit(0))
+dev, runs = C.c_int(), []
+ok(cu.cuDeviceGet(C.byref(dev), 0))
+for _ in range(2):
+    ctx = C.c_void_p()
+    ok(cu.cuCtxCreate_v2(C.byref(ctx), 0, dev))
+    runs.append(steps())
+    ok(cu.cuCtxDestroy_v2(ctx))
+runs.append(steps())     # the device's primary context
+for r in runs[1:]:
+    for a, b in zip(runs[0], r):
+        assert np.isfinite(b).all() and np.array_equal(a, b)
+print("same in every context")
+"""
+
+
+def test_one_cuda_context_after_another():
+    """The kernels' shared-memory limits belong to a CUDA context: a process that makes
+    another one current on the same device (or resets it) gets them set again."""
+    r = subprocess.run([sys.executable, "-c", CHILD, ROOT], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same in every context" in r.stdout, r.stdout + r.stderr
