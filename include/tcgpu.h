@@ -343,9 +343,11 @@ int tcgpu_tdm_solve_noalloc(int size, int nrhs, bool is_periodic, bool is_comple
 
 /* Self-test of the bounded waits inside the kernels. No counterpart in the
  * reference. Runs one block whose mbarrier wait can never complete (it expects
- * bytes no copy delivers): the wait must give up after its limit (about two
- * seconds of SM clock), the kernel report it and return, and the device stay
- * usable. Returns 0 when that happened; *seconds (if not NULL) = elapsed time. */
+ * bytes no copy delivers), then a small predict whose planes never arrive: the
+ * waits must give up after their limit (about two seconds of SM clock), the
+ * kernels report it and return, the predict without storing a field, and the
+ * device stay usable. Returns 0 when that happened; *seconds (if not NULL) =
+ * elapsed time. */
 int tcgpu_selftest_wait(double * seconds);
 
 /* free the device state that belongs to this fluid_t */

@@ -1352,25 +1352,42 @@ int tcgpu_statistics_mean_uy(const domain_t * domain, fluid_t * fluid, double * 
 }
 
 int tcgpu_selftest_wait(double * seconds) {
+  constexpr size_t K = PredictSelftest::KEPT;
+  PredictSelftest b{};
   unsigned * d = nullptr;
-  unsigned h = 0;
+  unsigned h[2] = {0, 0};
+  std::vector<unsigned char> kept(K * sizeof(double), 0);
   cudaStream_t st = nullptr;
   CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  if (cudaMalloc(&d, sizeof(unsigned)) != cudaSuccess) {
-    cudaStreamDestroy(st);
-    return fail("tcgpu_selftest_wait: cudaMalloc failed");
-  }
+  cudaError_t e = cudaMalloc(&d, 2 * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMalloc(&b.zeros, PredictSelftest::READ * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&b.kept, K * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&b.terms, PredictSelftest::FIELD * sizeof(double));
   const auto t0 = std::chrono::steady_clock::now();
-  cudaMemsetAsync(d, 0, sizeof(unsigned), st);
-  launch_wait_selftest(d, st);
-  cudaMemcpyAsync(&h, d, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-  const cudaError_t e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) {
+    cudaMemsetAsync(d, 0, 2 * sizeof(unsigned), st);
+    cudaMemsetAsync(b.zeros, 0, PredictSelftest::READ * sizeof(double), st);
+    cudaMemsetAsync(b.kept, 0xa5, K * sizeof(double), st);
+    launch_wait_selftest(d, st);
+    launch_predict_selftest(b, d + 1, st);
+    e = cudaGetLastError();
+    cudaMemcpyAsync(h, d, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(kept.data(), b.kept, K * sizeof(double), cudaMemcpyDeviceToHost, st);
+    const cudaError_t done = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = done;
+  }
   const auto t1 = std::chrono::steady_clock::now();
   cudaFree(d);
+  cudaFree(b.zeros);
+  cudaFree(b.kept);
+  cudaFree(b.terms);
   cudaStreamDestroy(st);
   if (seconds) *seconds = std::chrono::duration<double>(t1 - t0).count();
   if (e != cudaSuccess) return fail("tcgpu_selftest_wait: %s", cudaGetErrorString(e));
-  if (!(h & ST_TIMEOUT)) return fail("tcgpu_selftest_wait: the wait did not report giving up");
+  for (unsigned s : h)
+    if (!(s & ST_TIMEOUT)) return fail("tcgpu_selftest_wait: a wait did not report giving up");
+  for (unsigned char c : kept)
+    if (c != 0xa5) return fail("tcgpu_selftest_wait: a predict that gave up stored fields");
   return 0;
 }
 

@@ -240,6 +240,18 @@ void launch_xsolve(const Geo & g, const Bc & bc, const XFactors & xf, int rkstep
                    const FieldBufs & in, const FieldBufs & out, bool update, cudaStream_t st);
 // one CTA whose mbarrier wait can never complete: sets ST_TIMEOUT in *status
 void launch_wait_selftest(unsigned * status, cudaStream_t st);
+// a predict whose planes never arrive: sets ST_TIMEOUT in *status and writes no field
+struct PredictSelftest {
+  static constexpr int NX = 16, NY = 12, NZ = 4;   // two CTAs a plane, the second half empty
+  static constexpr size_t FIELD = (size_t)(NX + 2) * (NY + 2) * (NZ + 2);   // doubles (an even number)
+  static constexpr size_t READ = (size_t)NCOEF_TABLES * CSTRIDE;            // of zeros: the tables, more than a field
+  static constexpr size_t KEPT = 4 * FIELD;
+  static_assert(READ >= FIELD, "the fields are read from the same zeros");
+  double * zeros;   // READ
+  double * kept;    // KEPT
+  double * terms;   // FIELD: source terms of all variables, not looked at
+};
+void launch_predict_selftest(const PredictSelftest & b, unsigned * status, cudaStream_t st);
 void launch_xfactors(const XFactors & xf, const double * dtp, double nu, double kappa, cudaStream_t st);
 void launch_apply(const Geo & g, const Bc & bc, const FieldBufs & in, const FieldBufs & out, const DeltaSet & ds,
                   cudaStream_t st);

@@ -92,4 +92,29 @@ __global__ void wait_selftest_kernel(unsigned * status) {
 
 void launch_wait_selftest(unsigned * status, cudaStream_t st) { wait_selftest_kernel<<<1, 64, 0, st>>>(status); }
 
+// Self-test of the predict's way out: every plane announces 16 bytes more than its
+// copies bring, so no plane ever arrives, and every CTA must give up, store no field and
+// report ST_TIMEOUT. zeros: what the kernel reads, kept: the fields it would write.
+void launch_predict_selftest(const PredictSelftest & b, unsigned * status, cudaStream_t st) {
+  Geo g{};
+  g.nx = PredictSelftest::NX;
+  g.ny = PredictSelftest::NY;
+  g.nz = PredictSelftest::NZ;
+  constexpr size_t F = PredictSelftest::FIELD;
+  march::Args<double> A{};
+  A.g = g;
+  A.cf.tab = b.zeros;
+  A.in = FieldsT<double>{b.zeros, b.zeros, b.zeros, b.zeros, b.zeros, b.zeros};
+  A.out = FieldsT<double>{b.kept, b.kept + F, b.kept + 2 * F, nullptr, nullptr, b.kept + 3 * F};
+  for (int v = 0; v < 4; v++) {
+    A.ss.old_[v] = b.zeros;
+    A.ss.new_[v] = b.terms;
+  }
+  A.rkstep = 1;
+  A.mode = PREDICT_APPLY;
+  A.status = status;
+  A.lost = 16;
+  march::launch<0, double>(A, false, b.zeros, st);
+}
+
 }  // namespace tcgpu

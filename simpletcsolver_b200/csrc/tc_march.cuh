@@ -118,13 +118,18 @@ struct Args {
   DeltaSet ds;
   int rkstep, mode, KC;
   unsigned * status;
+  unsigned lost;   // bytes announced with every plane that no copy brings: 0 but in the self-test of the waits
 };
 
 __device__ __forceinline__ void mbar_arrive(unsigned long long * bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// bounded wait; after any wait of the CTA has given up, nobody waits any more
-// (the CTA runs to its end without storing anything)
+// Bounded wait of one thread; after any wait of the CTA has given up, nobody waits any
+// more: the CTA runs to its end, arriving as ever, without copying or storing fields any
+// more (source terms it still stores; they belong to a step that is reported as failed,
+// and a look at the flag before each store costs up to 3.5% of the kernel). The lanes of a
+// warp may find out at different times, so a branch on the flag holds no operation of a
+// whole warp (__syncwarp, shuffles) unless the warp has voted on it.
 __device__ __forceinline__ bool await(unsigned long long * bar, unsigned parity, volatile int * abort_flag) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
@@ -593,6 +598,7 @@ struct Copies {
     off = (unsigned)((f == 4 ? L::POFF : 0) + (size_t)o * es - (s - a) * es);
     total = bytes;
     for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
+    total += A.lost;
     next = x.k0 - 1;
     // the CTA's lines of a variable are consecutive in the packed layout; an even
     // number of lines before them starts them on a 16-byte boundary
@@ -607,8 +613,7 @@ struct Copies {
     const int m = next - x.k0 + 1, sl = m % L::NSLOT;
     if (next > x.k1) return;
     if (m >= L::NSLOT) await(bars.empty(sl), (unsigned)(m / L::NSLOT - 1) & 1u, abort_flag);
-    if (*abort_flag) return;
-    __syncwarp();
+    if (__any_sync(0xffffffffu, *abort_flag != 0)) return;
     if ((threadIdx.x & 31) == 0) mbar_expect_tx(bars.full(sl), total);
     __syncwarp();
     if (bytes) bulk_g2s(ring + (size_t)sl * L::SLOT + off, src, bytes, bars.full(sl));
@@ -627,14 +632,19 @@ struct Copies {
     old += old_step;
     next_old++;
   }
-  // No copy outlives the CTA: wait, bounded, for the latest fill of each slot and
-  // buffer (on the ordinary path the consumers wait for them too).
+  // No copy outlives the CTA: wait, one limit for all of them, for the latest fill of
+  // each slot and buffer (on the ordinary path the consumers wait for them too).
   __device__ __forceinline__ void drain(const Args<T> & A, const Box & x, const Bars<L> & bars) {
+    const long long t0 = clock64();
+    auto settle = [&](unsigned long long * bar, unsigned parity) {
+      while (!mbar_try_wait(bar, parity))
+        if (clock64() - t0 > kWaitCycles) return;
+    };
     for (int kp = next - L::NSLOT > x.k0 - 1 ? next - L::NSLOT : x.k0 - 1; kp < next; kp++)
-      mbar_wait(bars.full(slot_of<L>(kp, x.k0)), fill_of<L>(kp, x.k0));
-    if (TILE || A.rkstep == 0) return;
-    for (int ko = next_old - 2 > x.k0 ? next_old - 2 : x.k0; ko < next_old; ko++)
-      mbar_wait(bars.olds((ko - x.k0) & 1), (unsigned)((ko - x.k0) / 2) & 1u);
+      settle(bars.full(slot_of<L>(kp, x.k0)), fill_of<L>(kp, x.k0));
+    if constexpr (!TILE)
+      for (int ko = next_old - 2 > x.k0 ? next_old - 2 : x.k0; ko < next_old && A.rkstep != 0; ko++)
+        settle(bars.olds((ko - x.k0) & 1), (unsigned)((ko - x.k0) / 2) & 1u);
   }
 };
 
