@@ -505,7 +505,9 @@ def fp32_storage_arm(args, lib, d0, case, world, peak, value64):
     return out
 
 
-MODEL_BYTES_PER_CELL_STEP_PLANAR = 1512   # + y and z implicit solves and the increment round trip per substep
+# + per substep the y solves (increments read and written) and the z solves (increments
+# and fields read, fields written)
+MODEL_BYTES_PER_CELL_STEP_PLANAR = MODEL_BYTES_PER_CELL_STEP + 3 * (64 + 96)
 
 
 def planar_arm(args, lib, world, peak):

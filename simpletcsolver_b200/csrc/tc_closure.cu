@@ -555,9 +555,9 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) conv3_kernel(ConvArgs A) {
 // ring of NG plane slots interleaved per row, units [y][slot][co chunk][x], whose
 // first two slots are kept twice (NG, NG + 1), so a window of three never wraps.
 // Three accumulators (dx) of 3 COUT columns live in tensor memory for the whole
-// life of the CTA, zeroed first, so every MMA accumulates. A CTA takes an equal
-// contiguous share of the planes of all column tiles (ConvCursor) and writes its
-// raw partial sums, reduced afterwards by wgrad_reduce_kernel.
+// life of the CTA, zeroed first, so every MMA accumulates. A CTA strides over whole
+// items of a column tile and some planes (WgradCursor; the order of the sums follows
+// from it) and writes its raw partial sums, reduced afterwards by wgrad_reduce_kernel.
 //
 // Roles, meeting at mbarriers only: loader warps bring halo plane p and gradient
 // tile p + 1 of each step; one thread of the MMA warp issues a step's 24 MMAs,
@@ -654,7 +654,7 @@ __device__ __forceinline__ void load_wgrad_tile(char * tiles, const WgradArgs & 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(WG_THREADS, 1) conv3_wgrad_kernel(WgradArgs A) {
   using L = WgradLayout<CIN, COUT>;
-  constexpr int NS = L::NSW, NG = L::NG, CG = COUT / 8;
+  constexpr int NS = L::NSW, NG = L::NG;
   extern __shared__ __align__(128) char smw[];
   char * tiles = smw + L::GOFF;
   unsigned long long * full = reinterpret_cast<unsigned long long *>(smw + L::BAR);

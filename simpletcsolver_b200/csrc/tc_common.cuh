@@ -97,7 +97,7 @@ template <class T> __host__ __device__ inline int sline(const Geo & g, int n_i) 
 
 // periodic images of interior (j, k) in the one-layer halo, including the
 // corner written by the z exchange after the y exchange (src/halo.c:18-142);
-// ny, nz >= 2 (the FFTs require powers of two >= 4)
+// ny, nz >= 4
 template <typename F>
 __device__ inline void for_images(int j, int k, int ny, int nz, F && f) {
   const int jj = (j == 1) ? ny + 1 : (j == ny) ? 0 : -1;

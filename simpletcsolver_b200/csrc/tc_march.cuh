@@ -26,9 +26,9 @@
 // behind. The kernel moves 104 / 136 bytes a cell (the first / later substeps),
 // 2.2 / 2.8 ms at 256 x 1024 x 512 at the copy bandwidth, and its FP64 instructions
 // need about 1.2 ms of the FP64 pipe; at nx = 256 a plane of two lines takes a
-// solve warp about 4.6 thousand cycles: 2.1 the two solves (dependent FP64 and
-// shuffle latencies), 0.65 issuing copies, 0.55 the update, 0.36 the stores, the
-// rest waits. One CTA of 12 warps fits an SM: 8 field warps with both groups at
+// solve warp about 4.0 thousand cycles (clock64 around each part, 256 x 512 x 128):
+// 1.55 the two solves (dependent FP64 and shuffle latencies), 0.78 issuing copies,
+// 1.16 the update and the stores, 0.45 waits. One CTA of 12 warps fits an SM: 8 field warps with both groups at
 // 176 registers and 4 solve warps at 152, none spilling. 16 field warps at 96
 // registers spill and are slower (1.80 against 1.09 ms at 256 x 512 x 256), as are
 // solves whose scans run half as far (30.7 against 27.1 ps a cell). Per launch
@@ -469,7 +469,7 @@ __device__ __forceinline__ int spad(int e) { return e + e / E; }
 // zero where a level has no source lane, so a level is one shuffle and one
 // multiply-add. The factors of a lane stay in registers for all its lines; several
 // lines at a time (stride doubles apart) hide the chains' and the shuffles' latency.
-// Elements from n on have f = g = w = 0. Per plane of two 256-point lines: 1.9k
+// Elements from n on have f = g = w = 0. Per plane of two 256-point lines: 1.55k
 // cycles, against 4.2k with the factor rows read and multiplied out for each line.
 // SINGLE (FP32-storage contexts) keeps the former order of roundings: r_m w_m
 // first, f_m = -w_m l_m and g_m = -v_m with the rows' l, w, v (XFactors::single).

@@ -1,6 +1,6 @@
-// The right-hand sides of the marching predict kernel in FP32-storage contexts:
-// float arithmetic on the float fields (differences of the double p rounded once);
-// the increments, the radial solves and the update stay double. The order of every
+// The right-hand sides and increments of the marching predict kernel in FP32-storage
+// contexts: float arithmetic on the float fields (differences of the double p rounded
+// once); the increments are widened for the radial solves and the update, which are double. The order of every
 // rounding is part of the mode's results (a single-precision state has no room
 // below its rounding: another order of the same sums changes the last bit of
 // stored values, and through them the time step), so each cell keeps the plain

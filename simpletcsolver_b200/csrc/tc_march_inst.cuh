@@ -19,7 +19,8 @@ void launch_one(Args<T> A, const double * dtp, cudaStream_t st) {
   kernel<<<(unsigned)(columns * (A.g.nz / A.KC)), L::THREADS, L::BYTES, st>>>(A, dtp);
 }
 
-// warps per line by its length, and as many line pairs as make 12 to 16 field warps
+// warps per line by its length, line pairs, and 1 or 2 groups of field warps per line:
+// 4, 8 or 12 field warps, the fastest of the splits measured at each length
 #ifndef TC_MARCH_INSTANCES
 #define TC_MARCH_INSTANCES(X) X(1, 4, 1) X(2, 4, 1) X(3, 2, 2) X(4, 2, 1) X(6, 1, 2) X(8, 1, 1)
 #endif
